@@ -192,6 +192,18 @@ class Outputs(dict):
         self.owner = owner
 
 
+_stream = None
+
+
+def _program_stream():
+    """The program's simulation stream: every context's work runs on it in order, as the successive frames of one scene
+    do (a frame needs the one before it), so that a pass's time is a frame's and not a share of several at once."""
+    global _stream
+    if _stream is None:
+        _stream = torch.cuda.Stream()
+    return _stream
+
+
 class Scene:
     """A context with its fields loaded; closed with the object."""
 
@@ -201,7 +213,7 @@ class Scene:
         self.case = case
         self.cfg, f = _scene(case, seed)
         self.fields = f  # device inputs stay alive while the context may read them
-        self.stream = torch.cuda.Stream()
+        self.stream = _program_stream()
         self.frame = 0
         self.net = None
         sim = self.sim = smoke_b200.Simulation(smoke_b200.SmokeLibrary(), self.cfg, self.stream)
@@ -244,7 +256,7 @@ class Scenes:
 
     def __init__(self, cases, seed):
         self.members = [Scene(c, seed + 7919 * i) for i, c in enumerate(cases)]
-        self.batch = smoke_b200.Batch([m.sim for m in self.members])
+        self.batch = smoke_b200.Batch([m.sim for m in self.members], _program_stream())
 
     def __del__(self):
         if self.batch is not None:
