@@ -1,0 +1,55 @@
+"""The fixed-count CG solve of grids that fit on the chip (pcg_resident.cu) against the float64 oracle's CG
+(backend-cuda.cu:1788-1824), at the edges of its split: 32 x 8-cell columns, a block's range of planes crossing from one
+column into the next, one-cell and one-row remainder columns, both register variants and the ends of their ranges, periodic
+axes (halo words from the far side, a column that is its own neighbour) and solids.
+
+Tolerance: FP32 vectors, FP64 dot products and 10 iterations. An iteration rounds its four updates once each (eps = 6e-8) and
+the operator about seven times; carried through 10 iterations of growing search directions (at most a factor of ten) that is
+10 * 11 * 6e-8 * 10 < 1e-4 of the largest pressure.
+"""
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+import scenes
+import smoke_abi as abi
+import smoke_b200
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (8, 8, 8),       # one block, one plane row of a column
+    (33, 9, 16),     # remainder columns of one cell and one row
+    (32, 8, 40),     # a single column cut into blocks
+    (40, 24, 9),     # planes of two columns in one block
+    (31, 57, 23),
+    (65, 41, 48),
+    (96, 128, 96),   # 32 planes a block: the end of the middle variant
+    (128, 128, 128), # the large variant
+]
+
+
+@pytest.mark.parametrize("boundary", ["closed", "plume", "zout"])
+@pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
+@pytest.mark.parametrize("reduction", [abi.REDUCTION_FP32, abi.REDUCTION_FP64], ids=["fp32", "fp64"])
+def test_fixed_cg_on_chip_matches_oracle(smoke_lib, cuda_stream, shape, boundary, reduction):
+    cfg = scenes.make_config(*shape, boundary=boundary, mode=abi.LINEAR, pressure_iterations=10)
+    inp = scenes.random_inputs(cfg, seed=sum(shape), solids=shape[0] != 32)
+    sim = smoke_b200.Simulation(smoke_lib, cfg, cuda_stream)
+    keep = scenes.load_gpu(sim, inp)
+    sim.set_solver(abi.SOLVER_FIXED_CG, reduction)
+    with torch.cuda.stream(cuda_stream):
+        sim.step_stages(abi.STAGE_PRESSURE)
+    rhs = sim.snapshot([abi.VIEW_FLOW_PRESSURE_RHS])["pressure_rhs"]
+    p = sim.snapshot([abi.VIEW_FLOW_PRESSURE])["pressure"]
+    with torch.cuda.stream(cuda_stream):
+        sim.solve_pressure()  # the next launch's words carry other tags in the same buffers
+    again = sim.snapshot([abi.VIEW_FLOW_PRESSURE])["pressure"]
+    status = sim.solver_status()
+    sim.close()
+    del keep
+    x, _ = O.solve_pressure(cfg, inp["occupancy"], rhs, bits=64, mode=0)
+    assert status.iterations == 10 and status.status == abi.SOLVE_ITERATION_CAP
+    assert np.array_equal(p, again)
+    assert scenes.rel_err(p, x) < 1e-4

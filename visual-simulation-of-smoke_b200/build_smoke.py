@@ -7,6 +7,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -16,7 +17,7 @@ LIB = os.path.join(HERE, "libsmoke_b200.so")
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
-CU_SOURCES = ["step_kernels.cu", "pcg.cu", "mgsolve.cu", "noalloc.cu", "unet.cu"]
+CU_SOURCES = ["step_kernels.cu", "pcg.cu", "pcg_resident.cu", "mgsolve.cu", "noalloc.cu", "unet.cu"]
 CPP_SOURCES = ["context.cpp", "learned.cpp"]
 CLI = os.path.join(os.path.dirname(os.path.abspath(__file__)), "smoke_b200_benchmark")
 HEADERS = ["smoke_device.cuh", "launch.h", "config_check.h", "grid_sync.cuh", "march.cuh", "unet.h", "tcgen05.cuh", "pdl.cuh"]
@@ -47,21 +48,21 @@ def build(force: bool = False, verbose: bool = False) -> str:
     inc = [f"-I{p}" for p in INCLUDES]
     deps = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", h) for h in os.listdir(os.path.join(ROOT, "include"))]
     dep_time = _newest(deps + [os.path.abspath(__file__)])
-    objects = []
-    for src in CU_SOURCES:
+
+    def compile_one(src):
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src + ".o")
-        objects.append(o)
+        out = ""
         if force or not os.path.exists(o) or os.path.getmtime(o) < max(dep_time, os.path.getmtime(s)):
-            out = _run([NVCC, *NVCC_FLAGS, *inc, "-c", s, "-o", o])
+            out = _run([NVCC, *NVCC_FLAGS, *inc, "-c", s, "-o", o] if src.endswith(".cu") else ["g++", *CXX_FLAGS, *inc, f"-I{CUDA_HOME}/include", "-c", s, "-o", o])
+        return o, out
+
+    objects = []
+    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        for o, out in pool.map(compile_one, CU_SOURCES + CPP_SOURCES):
+            objects.append(o)
             if verbose and out:
                 print(out)
-    for src in CPP_SOURCES:
-        s = os.path.join(CSRC, src)
-        o = os.path.join(BUILD, src + ".o")
-        objects.append(o)
-        if force or not os.path.exists(o) or os.path.getmtime(o) < max(dep_time, os.path.getmtime(s)):
-            _run(["g++", *CXX_FLAGS, *inc, f"-I{CUDA_HOME}/include", "-c", s, "-o", o])
     if force or not os.path.exists(LIB) or os.path.getmtime(LIB) < _newest(objects):
         _run([NVCC, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB, *objects, "-cudart", "static", "-Xlinker", "--no-undefined"])
     # the benchmark CLI (loads the library, or any library exporting the ABI, at run time)

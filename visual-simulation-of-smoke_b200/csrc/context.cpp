@@ -160,6 +160,7 @@ struct SmokeSimulationContext_t {
         slots.push_back({reinterpret_cast<void**>(&fill_count), sizeof(uint32_t)});
         slots.push_back({reinterpret_cast<void**>(&anchor), sizeof(int32_t)});
         slots.push_back({reinterpret_cast<void**>(&control), sizeof(PcgControl)});
+        if (const size_t words = pcg_exchange_bytes(pcg_shape.resident)) slots.push_back({reinterpret_cast<void**>(&pcg.exchange), words});
         slots.push_back({reinterpret_cast<void**>(&mg_state), sizeof(MgState)});
         mg_work.part_stride = mg_partial_blocks(P.nx, P.ny, P.nz);
         slots.push_back({reinterpret_cast<void**>(&mg_work.part), static_cast<size_t>(kAccCount) * mg_work.part_stride * sizeof(double)});
@@ -578,7 +579,7 @@ SmokeSimulationResult smoke_simulation_create_context_cuda(const SmokeSimulation
         check(cudaGetDevice(&dev), "device");
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
         ctx->fill_blocks = sms * 4;
-        check(pcg_launch_shape(&ctx->pcg_shape), "solver launch shape");
+        check(pcg_launch_shape(ctx->P, &ctx->pcg_shape), "solver launch shape");
         ctx->allocate();
         cudaStream_t s = ctx->stream;
         check(cudaMemsetAsync(ctx->arena, 0, ctx->arena_bytes, s), "zero arena");

@@ -130,6 +130,7 @@ struct PcgControl {
     unsigned int pad2[28];
     double totals[3][kPcgSumCopies][16];  // 4 sums per copy, one 128-byte line per copy
     PcgStatusDevice status;
+    unsigned int epoch;  // tag of the last exchange of the resident kernel's launches so far (never reset)
 };
 constexpr size_t kPcgControlResetBytes = offsetof(PcgControl, status);
 
@@ -140,14 +141,22 @@ struct PcgWork {
     float* p;
     float* e;      // FP32 correction iterate of a refinement pass
     double* x64;   // FP64 solution accumulator (refinement); kept between steps as the warm start
-    double* part;  // per-block partial sums of the dot products, [kAccCount][part_stride] (FP64)
-    uint32_t part_stride;  // blocks of the largest level-0 grid (mg_partial_blocks)
+    unsigned long long* exchange;  // the resident kernel's words (pcg_exchange_bytes; null: the streaming kernel runs)
 };
-// Blocks of the largest grid a level-0 kernel of the multigrid solve launches on an nx x ny x nz grid (one
-// 32 x 4 x 2 tile per block): the length of each accumulator's row of per-block partial sums.
-uint32_t mg_partial_blocks(int nx, int ny, int nz);
+
+// The resident kernel's split: ncx x ncy columns of 32 x 8 cells, `total` (column, plane) units over `blocks` blocks of at
+// most `planes` each (blocks = 0: the grid does not fit on the chip and the streaming kernel runs).
+struct PcgResidentPlan {
+    int ncx, ncy;
+    uint32_t total;
+    int blocks, planes;
+};
+constexpr int kPcgResidentPlanes = 70;  // 231,680 bytes of shared memory, and 140 registers for a thread's w and s
+PcgResidentPlan pcg_resident_plan(int nx, int ny, int nz, int sms);
+size_t pcg_exchange_bytes(const PcgResidentPlan& plan);
 
 struct PcgLaunchShape {
+    PcgResidentPlan resident;
     int blocks;
     int threads;
     int grid;  // kPcgGridCount code: the persistent grid is the resident blocks divided by 1 << grid
@@ -255,7 +264,9 @@ cudaError_t enqueue_mg_solve(const MgSolveArgs& args, bool fp64, PcgStatusDevice
 cudaError_t run_mg_solve_eager(const MgSolveArgs& args, bool fp64, PcgStatusDevice* status_out, cudaStream_t s);
 
 // Picks the persistent grid (all blocks co-resident) for the current device.
-cudaError_t pcg_launch_shape(PcgLaunchShape* out);
+cudaError_t pcg_launch_shape(const StepParams& P, PcgLaunchShape* out);
+// The fixed-count solve with its state on the chip (pcg_resident.cu).
+cudaError_t launch_pcg_resident(const StepParams& P, const PcgSettings& S, const PcgResidentPlan& plan, const uint16_t* codes, const float* b, float* x, const PcgWork& work, PcgControl* ctl, cudaStream_t s);
 // Enqueues: reset of the control header, then the cooperative solver launch.
 cudaError_t launch_pcg(const StepParams& P, const PcgSettings& S, const PcgLaunchShape& shape, const uint16_t* codes, const float* b, float* x, PcgWork work, PcgControl* ctl, cudaStream_t s);
 

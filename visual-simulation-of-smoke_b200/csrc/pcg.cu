@@ -413,11 +413,12 @@ cudaError_t launch_one(const StepParams& P, const PcgSettings& S, int grid, cons
 
 }  // namespace
 
-cudaError_t pcg_launch_shape(PcgLaunchShape* out) {
+cudaError_t pcg_launch_shape(const StepParams& P, PcgLaunchShape* out) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
+    out->resident = pcg_resident_plan(P.nx, P.ny, P.nz, sms);
     out->blocks = sms;
     out->threads = kThreads;
     out->grid = 0;
@@ -432,6 +433,9 @@ cudaError_t launch_variant(const StepParams& P, const PcgSettings& S, int g, con
 }
 
 cudaError_t launch_pcg(const StepParams& P, const PcgSettings& S, const PcgLaunchShape& shape, const uint16_t* codes, const float* b, float* x, PcgWork work, PcgControl* ctl, cudaStream_t s) {
+    // fixed-count solves of grids that fit on the chip run there (FP64 sums take 2 KB of shared memory, the space of the last
+    // plane); the launch shape's knobs are this file's kernel's
+    if (S.fixed && !S.jacobi && shape.resident.blocks > 0 && work.exchange != nullptr && (!S.fp64 || shape.resident.planes < kPcgResidentPlanes)) return launch_pcg_resident(P, S, shape.resident, codes, b, x, work, ctl, s);
     return shape.regs ? launch_variant<4>(P, S, shape.grid, codes, b, x, work, ctl, s) : launch_variant<1>(P, S, shape.grid, codes, b, x, work, ctl, s);
 }
 
