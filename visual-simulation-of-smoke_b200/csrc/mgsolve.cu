@@ -112,12 +112,14 @@ __device__ __forceinline__ R stencil_xyz(const MgLevel& L, uint32_t q, int x, in
     return acc;
 }
 
-// Masked 7-point stencil from preloaded values: diag * v0 - sum of vn[e] over the code's active neighbour bits.
-__device__ __forceinline__ float masked_stencil(uint16_t code, float v0, const float vn[6]) {
-    float acc = diagf(code) * v0;
+// Masked 7-point stencil from preloaded values: diag * v0 - sum of vn[e] over the code's active neighbour bits. The
+// roundings are spelled out, so that every kernel forms the same value whatever the compiler contracts around it (a learned
+// solve carries an ulp here through the network's BF16 into its whole path).
+__device__ __forceinline__ float masked_stencil(uint16_t code, float v0, const float* vn) {
+    float acc = __fmul_rn(diagf(code), v0);
 #pragma unroll
     for (int e = 0; e < 6; ++e)
-        if (code & (1u << e)) acc -= vn[e];
+        if (code & (1u << e)) acc = __fsub_rn(acc, vn[e]);
     return acc;
 }
 
@@ -302,151 +304,173 @@ __device__ __forceinline__ float restrict_tile(float c, const MgLevel& C, const 
 }
 
 // ---------------------------------------------------------------------------------------------- level-0 z-march
-// The level-0 passes of an iteration (update, smoothing, p/q) march in z. Level 0 is cut into MX x MY = 32 x 8
-// columns; each block owns a balanced range of (column, plane pair) units and walks its column segments in z, two
-// planes per unit. Thread (tx, ty) owns one cell of the column plane, and a warp holds two y rows of 16 x cells
-// (lanes 0-15 row 2k, lanes 16-31 row 2k + 1), so the 2 x 2 x 2 children of a coarse cell are a lane pair (^1), a
-// half-warp pair (^16) and two consecutive planes: the restriction is two shuffles and a register. The value whose
-// stencil a pass takes is formed once per cell and plane. The 32 x 8 plane and its 84-cell halo go through a
-// three-plane ring in shared memory (the in-plane neighbours); the column's own -z / +z values stay in registers.
-// The loads of plane z + 2 are issued before plane z is computed; one __syncthreads per plane.
-constexpr int MX = 32, MY = 8, MPX = MX + 2, MPY = MY + 2;
-constexpr int kMPlane = MPX * MPY;
-constexpr int kMHalo = kMPlane - MX * MY;
-static_assert(MX * MY == kThreads && kMHalo <= kThreads, "one column cell per thread, at most one halo slot");
+// The level-0 passes of an iteration (update, smoothing, p/q) march in z, a warp by itself: it owns a column of 32 x 4
+// cells (MR = 4; 32 x 2 on small levels, march_rows), lane x, MR rows in each thread, and walks it plane by plane without shared memory or barriers. The value whose
+// stencil a pass takes is formed once per cell and plane for the MR rows and the row on either side (the neighbouring
+// warp's rows, an L1 hit), the x neighbours come by shuffle (the two cells beyond the warp's ends from 2 MR lanes that
+// load them), the -z / +z values stay in registers. The loads of plane z + 2 are issued before plane z is computed: about
+// 29 a thread, four times those of a march with one cell per thread, which waited for its loads at a block barrier every
+// plane. The 2 x 2 x 2 children of a coarse cell are a lane pair, two rows of a thread and two consecutive planes.
+// A block's 8 warps tile wx x wy such columns (march_shape); each block owns a balanced range of (tile, plane pair) units.
+constexpr int kMarchWarps = kThreads / 32;
 
 struct MarchUnits {
-    int ncx, ncy, nzu;  // columns along x and y, plane pairs along z
+    int wx, wy;         // warps of a block along x and y
+    int ncx, ncy, nzu;  // tiles along x and y, plane pairs along z
     uint32_t total;     // ncx * ncy * nzu
 };
+// The arrangement of a block's warps that pads the level least (the tallest of equals: halo rows are then L1 hits).
+template <int MR>
 __host__ __device__ inline MarchUnits march_units(const MgLevel& L) {
-    MarchUnits u;
-    u.ncx = (L.nx + MX - 1) / MX;
-    u.ncy = (L.ny + MY - 1) / MY;
+    MarchUnits u{};
+    uint64_t least = ~0ull;
+    for (int wy = kMarchWarps; wy >= 1; wy >>= 1) {
+        const int wx = kMarchWarps / wy;
+        const int ncx = (L.nx + 32 * wx - 1) / (32 * wx), ncy = (L.ny + MR * wy - 1) / (MR * wy);
+        const uint64_t cells = static_cast<uint64_t>(ncx) * wx * static_cast<uint64_t>(ncy) * wy;
+        if (cells < least) {
+            least = cells;
+            u.wx = wx;
+            u.wy = wy;
+            u.ncx = ncx;
+            u.ncy = ncy;
+        }
+    }
     u.nzu = (L.nz + 1) / 2;
     u.total = static_cast<uint32_t>(u.ncx) * static_cast<uint32_t>(u.ncy) * static_cast<uint32_t>(u.nzu);
     return u;
 }
 
-// A ring slot: the in-plane cell it holds (wrapped across periodic edges), if that cell exists.
-struct MSlot {
-    int slot;
-    uint32_t off;  // y * nx + x of the cell
-    bool load;
-};
-__device__ __forceinline__ MSlot march_slot(const MgLevel& L, const int* per, int x0, int y0, int hx, int hy) {
-    MSlot s;
-    s.slot = (hy + 1) * MPX + hx + 1;
-    int x = x0 + hx, y = y0 + hy;
-    bool ok = true;
-    if (x < 0 || x >= L.nx) {
-        if (per[0]) x = wrapi(x, L.nx);
-        else ok = false;
-    }
-    if (y < 0 || y >= L.ny) {
-        if (per[1]) y = wrapi(y, L.ny);
-        else ok = false;
-    }
-    s.load = ok;
-    s.off = ok ? static_cast<uint32_t>(y) * static_cast<uint32_t>(L.nx) + static_cast<uint32_t>(x) : 0u;
-    return s;
+// Coordinate v within [-1, ...] of an axis of n cells: wrapped on a periodic axis; false when there is no such cell.
+__device__ __forceinline__ bool march_wrap(int& v, int n, int per) {
+    if (v >= 0 && v < n) return true;
+    if (!per) return false;
+    v = wrapi(v, n);
+    return true;
 }
 
 // March over this block's units of level L. Per plane z of a segment:
-//   lo(ok, q) -> Own, lh(ok, q) -> Halo       loads of the own cell / the halo slot (zeros when !ok)
-//   uo(Own), uh(Halo) -> float                 the value whose stencil is taken (into the ring)
-//   cell(out, q, Own, um1, u0, u1, plane, slot) -> float
-//       the own cell's work at plane z (out: the cell is inside the level; um1 / u1 its -z / +z values, plane the
-//       ring plane of z); called by every thread. RESTRICT: its result (0 outside the level) is the cell's residual,
-//       summed over the 2 x 2 x 2 children into C.r, in restrict_tile's order.
-template <bool RESTRICT, class Own, class Halo, class LO, class LH, class UO, class UH, class CellF>
-__device__ __forceinline__ void march0(const MgLevel& L, const int* per, const MgLevel& C, float (*ring)[kMPlane], LO&& lo, LH&& lh, UO&& uo, UH&& uh, CellF&& cell) {
-    const MarchUnits U = march_units(L);
+//   lh(ok, q) -> Halo                          loads of what the stencil's value is formed from (zeros when !ok)
+//   uh(Halo, Keep&) -> float                   that value; Keep holds what the own cell's work needs of the loads
+//   lo(ok, q) -> Own                           further loads of the own cell
+//   cell(q, Keep, Own, u0, un) -> float        the own cell's work at plane z (un: its -x +x -y +y -z +z values); called for
+//       cells of the level. RESTRICT: its result is the cell's residual, summed over the 2 x 2 x 2 children into C.r, in
+//       restrict_tile's order.
+template <int MR, bool RESTRICT, class Halo, class Keep, class Own, class LH, class UH, class LO, class CellF>
+__device__ __forceinline__ void march0(const MgLevel& L, const int* per, const MgLevel& C, LH&& lh, UH&& uh, LO&& lo, CellF&& cell) {
+    constexpr int MH = MR + 2;  // a thread's rows and the halo rows
+    const MarchUnits U = march_units<MR>(L);
     const uint32_t a = static_cast<uint32_t>((static_cast<uint64_t>(blockIdx.x) * U.total) / gridDim.x);
     const uint32_t b = static_cast<uint32_t>((static_cast<uint64_t>(blockIdx.x + 1) * U.total) / gridDim.x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tx = (lane & 15) + 16 * (warp & 1), ty = (lane >> 4) + 2 * (warp >> 1);
-    const bool halo = threadIdx.x < kMHalo;
-    int hx = 0, hy = 0;
-    if (halo) {
-        const int h = threadIdx.x;
-        if (h < MPX) {
-            hx = h - 1;
-            hy = -1;
-        } else if (h < 2 * MPX) {
-            hx = h - MPX - 1;
-            hy = MY;
-        } else if (h < 2 * MPX + MY) {
-            hx = -1;
-            hy = h - 2 * MPX;
-        } else {
-            hx = MX;
-            hy = h - 2 * MPX - MY;
-        }
-    }
+    const int wx = warp % U.wx, wy = warp / U.wx;
     const uint32_t slab = static_cast<uint32_t>(L.nx) * static_cast<uint32_t>(L.ny);
     uint32_t u = a;
     while (u < b) {
-        const uint32_t col = u / static_cast<uint32_t>(U.nzu);
-        const int zu = static_cast<int>(u - col * static_cast<uint32_t>(U.nzu));
+        const uint32_t tile = u / static_cast<uint32_t>(U.nzu);
+        const int zu = static_cast<int>(u - tile * static_cast<uint32_t>(U.nzu));
         const int zub = zu + static_cast<int>(min(static_cast<uint32_t>(U.nzu - zu), b - u));
         u += static_cast<uint32_t>(zub - zu);
         const int za = 2 * zu, zb = min(L.nz, 2 * zub);
-        const int x0 = static_cast<int>(col % static_cast<uint32_t>(U.ncx)) * MX, y0 = static_cast<int>(col / static_cast<uint32_t>(U.ncx)) * MY;
-        const MSlot so = march_slot(L, per, x0, y0, tx, ty);
-        const MSlot sh = march_slot(L, per, x0, y0, hx, hy);
-        const bool out = x0 + tx < L.nx && y0 + ty < L.ny;
+        const int xw = (static_cast<int>(tile % static_cast<uint32_t>(U.ncx)) * U.wx + wx) * 32;   // the warp's first cell
+        const int yw = (static_cast<int>(tile / static_cast<uint32_t>(U.ncx)) * U.wy + wy) * MR;  // and row
+        if (xw >= L.nx || yw >= L.ny) continue;  // uniform over the warp
+        const int x = xw + lane;
+        int xl = x;
+        const bool x_ok = march_wrap(xl, L.nx, per[0]);
+        // rows yw - 1 .. yw + MR (bit r of row_ok: there is such a row)
+        uint32_t off[MH], row_ok = 0;
+#pragma unroll
+        for (int r = 0; r < MH; ++r) {
+            int y = yw - 1 + r;
+            const bool ok = march_wrap(y, L.ny, per[1]);
+            row_ok |= (ok && x_ok ? 1u : 0u) << r;
+            off[r] = ok ? static_cast<uint32_t>(y) * static_cast<uint32_t>(L.nx) + static_cast<uint32_t>(x_ok ? xl : 0) : 0u;
+        }
+        // lanes 0 .. MR - 1: the cell left of the warp in row lane; lanes MR .. 2 MR - 1: the cell right of it in row lane - MR
+        int xe = lane < MR ? xw - 1 : xw + 32, ye = yw + (lane & (MR - 1));
+        const bool edge_ok = lane < 2 * MR && march_wrap(xe, L.nx, per[0]) && ye < L.ny;
+        const uint32_t edge_off = edge_ok ? static_cast<uint32_t>(ye) * static_cast<uint32_t>(L.nx) + static_cast<uint32_t>(xe) : 0u;
+        const bool out_x = x < L.nx;
+        const int rows = min(MR, L.ny - yw);
         // plane z's offset (wrapped across a periodic z edge); false outside a non-periodic level
         auto zbase = [&](int z, uint32_t& base) {
-            if (z < 0 || z >= L.nz) {
-                if (!per[2]) return false;
-                z = wrapi(z, L.nz);
-            }
-            base = static_cast<uint32_t>(z) * slab;
-            return true;
+            const bool ok = march_wrap(z, L.nz, per[2]);
+            base = ok ? static_cast<uint32_t>(z) * slab : 0u;
+            return ok;
         };
-        auto fetch = [&](int z, Own& od, Halo& hd, bool with_halo) {
-            uint32_t base = 0;
+        Halo h[MH], he;
+        Own o0[MR], o1[MR];
+        Keep k0[MR], k1[MR], drop;
+        float um1[MR], u0[MH], u1[MH], e0, e1;
+        auto fetch = [&](int z) {  // the halo loads of plane z
+            uint32_t base;
             const bool ok = zbase(z, base);
-            od = lo(ok && so.load, base + so.off);
-            if (with_halo && halo) hd = lh(ok && sh.load, base + sh.off);
+#pragma unroll
+            for (int r = 0; r < MH; ++r) h[r] = lh(ok && (row_ok >> r & 1u), base + off[r]);
+            he = lh(ok && edge_ok, base + edge_off);
         };
-        Own om1, o0, o1, o2;
-        Halo hunused, h0, h1, h2;
-        fetch(za - 1, om1, hunused, false);
-        fetch(za, o0, h0, true);
-        fetch(za + 1, o1, h1, true);
-        float um1 = uo(om1), u0 = uo(o0);
-        ring[za % 3][so.slot] = u0;
-        if (halo) ring[za % 3][sh.slot] = uh(h0);
-        float pair = 0.0f;
+        auto fetch_own = [&](int z, Own* o) {  // z inside the level
+#pragma unroll
+            for (int r = 0; r < MR; ++r) o[r] = lo(out_x && r < rows, static_cast<uint32_t>(z) * slab + off[r + 1]);
+        };
+        {
+            uint32_t base;
+            const bool ok = zbase(za - 1, base);
+#pragma unroll
+            for (int r = 0; r < MR; ++r) h[r] = lh(ok && (row_ok >> (r + 1) & 1u), base + off[r + 1]);
+#pragma unroll
+            for (int r = 0; r < MR; ++r) um1[r] = uh(h[r], drop);
+        }
+        fetch(za);
+        fetch_own(za, o0);
+#pragma unroll
+        for (int r = 0; r < MH; ++r) u0[r] = uh(h[r], r >= 1 && r <= MR ? k0[r - 1] : drop);
+        e0 = uh(he, drop);
+        fetch(za + 1);
+        float pair[MR / 2] = {};
         for (int z = za; z < zb; ++z) {
-            if (z + 2 <= zb) fetch(z + 2, o2, h2, true);
-            const float u1 = uo(o1);
-            ring[(z + 1) % 3][so.slot] = u1;
-            if (halo) ring[(z + 1) % 3][sh.slot] = uh(h1);
-            __syncthreads();
-            const float res = cell(out, static_cast<uint32_t>(z) * slab + so.off, o0, um1, u0, u1, ring[z % 3], so.slot);
+#pragma unroll
+            for (int r = 0; r < MH; ++r) u1[r] = uh(h[r], r >= 1 && r <= MR ? k1[r - 1] : drop);
+            e1 = uh(he, drop);
+            if (z + 1 < zb) {
+                fetch(z + 2);
+                fetch_own(z + 1, o1);
+            }
+            float res[MR];
+#pragma unroll
+            for (int r = 0; r < MR; ++r) {
+                const float left = __shfl_up_sync(0xffffffffu, u0[r + 1], 1), right = __shfl_down_sync(0xffffffffu, u0[r + 1], 1);
+                const float le = __shfl_sync(0xffffffffu, e0, r), re = __shfl_sync(0xffffffffu, e0, MR + r);
+                const float un[6] = {lane == 0 ? le : left, lane == 31 ? re : right, u0[r], u0[r + 2], um1[r], u1[r + 1]};
+                res[r] = out_x && r < rows ? cell(static_cast<uint32_t>(z) * slab + off[r + 1], k0[r], o0[r], u0[r + 1], un) : 0.0f;
+            }
             if (RESTRICT) {
-                // restrict_tile's association: ((a + b) + c) + d over the x pairs a, b (even plane, rows 2Y, 2Y + 1)
-                // and c, d (odd plane); the writer is the even-x lane of row 2Y
-                const float xs = res + __shfl_xor_sync(0xffffffffu, res, 1);
-                const float other = __shfl_xor_sync(0xffffffffu, xs, 16);
+                // restrict_tile's association: ((a + b) + c) + d over the x pairs a, b (even plane, rows 2Y, 2Y + 1) and c, d
+                // (odd plane); the even lanes write
                 const bool last = (z & 1) != 0 || z == L.nz - 1;
-                if ((z & 1) == 0) pair = xs + other;
-                else pair = (pair + xs) + other;
-                if (last && (tx & 1) == 0 && (ty & 1) == 0) {
-                    const int X = (x0 + tx) >> 1, Y = (y0 + ty) >> 1, Z = z >> 1;
-                    if (X < C.nx && Y < C.ny) C.r[lidx(C, X, Y, Z)] = pair;
+#pragma unroll
+                for (int j = 0; j < MR / 2; ++j) {
+                    const float c0 = res[2 * j] + __shfl_xor_sync(0xffffffffu, res[2 * j], 1);
+                    const float c1 = res[2 * j + 1] + __shfl_xor_sync(0xffffffffu, res[2 * j + 1], 1);
+                    if ((z & 1) == 0) pair[j] = c0 + c1;
+                    else pair[j] = (pair[j] + c0) + c1;
+                    if (last && (lane & 1) == 0) {
+                        const int X = x >> 1, Y = (yw >> 1) + j;
+                        if (X < C.nx && Y < C.ny) C.r[lidx(C, X, Y, z >> 1)] = pair[j];
+                    }
                 }
             }
-            um1 = u0;
-            u0 = u1;
-            o0 = o1;
-            o1 = o2;
-            h1 = h2;
+#pragma unroll
+            for (int r = 0; r < MR; ++r) {
+                um1[r] = u0[r + 1];
+                k0[r] = k1[r];
+                o0[r] = o1[r];
+            }
+#pragma unroll
+            for (int r = 0; r < MH; ++r) u0[r] = u1[r];
+            e0 = e1;
         }
-        __syncthreads();
     }
 }
 
@@ -505,12 +529,11 @@ __global__ void __launch_bounds__(kThreads) mg_setup_kernel(const __grid_constan
 // initial = 1: the pass's first round (alpha = 0, no iteration counted). The last block tests convergence, flips
 // the buffer parity and sets the loop condition `cond`: continue unless stopped, and (net_loop = 1, the loop of a
 // learned solve whose body runs the network) unless the next iteration goes without the network.
-// z-march: the ring holds w D^-1 (r - alpha q) of every cell (the pre-smoothed zp on active cells; the stencil's
+// z-march: the value is w D^-1 (r - alpha q) of every cell (the pre-smoothed zp on active cells; the stencil's
 // mask never reaches the others).
-template <typename T, bool LEARNED>
+template <typename T, bool LEARNED, int MR>
 __global__ void __launch_bounds__(kThreads) mg_update_kernel(const __grid_constant__ MgSolveArgs A, int initial, cudaGraphConditionalHandle cond, int in_graph, int net_loop) {
     pdl_begin();
-    __shared__ float ring[3][kMPlane];
     const MgLevel& L0 = A.H.L[0];
     MgState* st = A.st;
     const bool skip = st->halt || st->fail;  // uniform over the grid
@@ -521,29 +544,19 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(const __grid_consta
         const float* r = A.W.r[par];
         float* rn_out = A.W.r[par ^ 1];
         const float* pn = A.W.p[par ^ 1];
-        struct Own {
-            uint32_t code;
-            float r, q, p, e;
-        };
         struct Halo {
             uint32_t code;
             float r, q;
         };
-        march0<true, Own, Halo>(
-            L0, A.H.fper, A.H.L[1], ring,
-            [&](bool ok, uint32_t q) {
-                Own d{0u, 0.0f, 0.0f, 0.0f, 0.0f};
-                if (ok) {
-                    d.code = L0.code[q];
-                    d.r = r[q];
-                    d.q = A.W.q[q];
-                    if (!initial) {
-                        d.p = pn[q];
-                        d.e = A.e[q];
-                    }
-                }
-                return d;
-            },
+        struct Keep {
+            uint32_t code;
+            float rn;
+        };
+        struct Own {
+            float p, e;
+        };
+        march0<MR, true, Halo, Keep, Own>(
+            L0, A.H.fper, A.H.L[1],
             [&](bool ok, uint32_t q) {
                 Halo d{0u, 0.0f, 0.0f};
                 if (ok) {
@@ -553,16 +566,25 @@ __global__ void __launch_bounds__(kThreads) mg_update_kernel(const __grid_consta
                 }
                 return d;
             },
-            [&](const Own& d) { return wdiag(static_cast<uint16_t>(d.code)) * (d.r - a * d.q); },
-            [&](const Halo& d) { return wdiag(static_cast<uint16_t>(d.code)) * (d.r - a * d.q); },
-            [&](bool out, uint32_t q, const Own& d, float um1, float u0, float u1, const float* pl, int s) {
-                if (!out) return 0.0f;
-                const uint16_t code = static_cast<uint16_t>(d.code);
-                const float rn = d.r - a * d.q;
+            [&](const Halo& d, Keep& k) {
+                k.code = d.code;
+                k.rn = d.r - a * d.q;
+                return wdiag(static_cast<uint16_t>(d.code)) * k.rn;
+            },
+            [&](bool ok, uint32_t q) {
+                Own d{0.0f, 0.0f};
+                if (ok && !initial) {
+                    d.p = pn[q];
+                    d.e = A.e[q];
+                }
+                return d;
+            },
+            [&](uint32_t q, const Keep& k, const Own& d, float u0, const float* un) {
+                const uint16_t code = static_cast<uint16_t>(k.code);
+                const float rn = k.rn;
                 float zp = 0.0f, res = 0.0f;
                 if (active(code)) {
                     zp = u0;
-                    const float un[6] = {pl[s - 1], pl[s + 1], pl[s - MPX], pl[s + MPX], um1, u1};
                     res = 0.5f * (rn - masked_stencil(code, zp, un));
                 }
                 L0.zp[q] = zp;
@@ -752,40 +774,36 @@ __global__ void __launch_bounds__(kThreads) mg_smooth_kernel(const __grid_consta
 // Level-0 post-smoothing (z-march): z = zp + w D^-1 (r - A zp) on active cells, 0 elsewhere, into t; with DOTS,
 // (z, r) and (z, q), and the last block computes beta (0 on a pass's first iteration). DOTS = false (a learned
 // solve's iteration with the network): z only; the network's correction and the dot products follow.
-template <typename T, bool DOTS>
+template <typename T, bool DOTS, int MR>
 __global__ void __launch_bounds__(kThreads) mg_smooth0_kernel(const __grid_constant__ MgSolveArgs A) {
     pdl_begin();
-    __shared__ float ring[3][kMPlane];
     const MgLevel& F = A.H.L[0];
     MgState* st = A.st;
     const float* r = A.W.r[st->parity];
     T zr = 0, zq = 0;
+    struct None {};
     struct Own {
         uint32_t code;
-        float s, r, q;
+        float r, q;
     };
-    march0<false, Own, float>(
-        F, A.H.fper, F, ring,
+    march0<MR, false, float, None, Own>(
+        F, A.H.fper, F,
+        [&](bool ok, uint32_t q) { return ok ? F.zp[q] : 0.0f; },
+        [&](float v, None&) { return v; },
         [&](bool ok, uint32_t q) {
-            Own d{0u, 0.0f, 0.0f, 0.0f};
+            Own d{0u, 0.0f, 0.0f};
             if (ok) {
                 d.code = F.code[q];
-                d.s = F.zp[q];
                 d.r = r[q];
                 if (DOTS) d.q = A.W.q[q];
             }
             return d;
         },
-        [&](bool ok, uint32_t q) { return ok ? F.zp[q] : 0.0f; },
-        [&](const Own& d) { return d.s; },
-        [&](float v) { return v; },
-        [&](bool out, uint32_t q, const Own& d, float um1, float u0, float u1, const float* pl, int s) {
-            if (!out) return 0.0f;
+        [&](uint32_t q, None, const Own& d, float u0, const float* un) {
             const uint16_t code = static_cast<uint16_t>(d.code);
             float z = 0.0f;
             if (active(code)) {
-                const float sn[6] = {pl[s - 1], pl[s + 1], pl[s - MPX], pl[s + MPX], um1, u1};
-                z = u0 + wdiag(code) * (d.r - masked_stencil(code, u0, sn));
+                z = u0 + wdiag(code) * (d.r - masked_stencil(code, u0, un));
                 if (DOTS) {
                     zr += static_cast<T>(z) * static_cast<T>(d.r);
                     zq += static_cast<T>(z) * static_cast<T>(d.q);
@@ -925,48 +943,43 @@ __global__ void __launch_bounds__(kThreads) mg_net_gamma_kernel(const __grid_con
 // on active cells (z = z_V in iterations without the network). The network supplies the smooth part of the
 // correction; the Jacobi step removes the rough part of its error (BF16 output, fitting noise and the prolongation),
 // which the energy norm the FCG minimises would amplify. Then (z, r) and (z, q), and the last block computes beta (0
-// on a pass's first iteration), as level 0's smoothing does for the V-cycle alone. z-march: the ring holds gamma N
+// on a pass's first iteration), as level 0's smoothing does for the V-cycle alone. z-march of gamma N
 // (32 -> 25 us against the per-cell form at 128^3).
-template <typename T>
+template <typename T, int MR>
 __global__ void __launch_bounds__(kThreads) mg_net_add_kernel(const __grid_constant__ MgSolveArgs A, const float* __restrict__ N) {
     pdl_begin();
-    __shared__ float ring[3][kMPlane];
     const MgLevel& F = A.H.L[0];
     MgState* st = A.st;
     const bool use_net = st->net_off == 0;
     const float g = use_net ? static_cast<float>(st->net_gamma) : 0.0f;
     const float* r = A.W.r[st->parity];
     T zr = 0, zq = 0;
+    struct None {};
     struct Own {
         uint32_t code;
-        float n, t, rv, r, q;
+        float t, rv, r, q;
     };
-    march0<false, Own, float>(
-        F, A.H.fper, F, ring,
+    march0<MR, false, float, None, Own>(
+        F, A.H.fper, F,
+        [&](bool ok, uint32_t q) { return ok && use_net ? N[q] : 0.0f; },
+        [&](float v, None&) { return v * g; },
         [&](bool ok, uint32_t q) {
-            Own d{0u, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            Own d{0u, 0.0f, 0.0f, 0.0f, 0.0f};
             if (ok) {
                 d.code = F.code[q];
                 d.t = F.t[q];
                 d.r = r[q];
                 d.q = A.W.q[q];
-                if (use_net) {
-                    d.n = N[q];
-                    d.rv = F.zp[q];
-                }
+                if (use_net) d.rv = F.zp[q];
             }
             return d;
         },
-        [&](bool ok, uint32_t q) { return ok && use_net ? N[q] : 0.0f; },
-        [&](const Own& d) { return d.n * g; },
-        [&](float v) { return v * g; },
-        [&](bool out, uint32_t q, const Own& d, float um1, float u0, float u1, const float* pl, int s) {
+        [&](uint32_t q, None, const Own& d, float u0, const float* un) {
             const uint16_t code = static_cast<uint16_t>(d.code);
-            if (!out || !active(code)) return 0.0f;  // t stays 0 there
+            if (!active(code)) return 0.0f;  // t stays 0 there
             float z = d.t;
             if (use_net) {
-                const float nn[6] = {pl[s - 1], pl[s + 1], pl[s - MPX], pl[s + MPX], um1, u1};
-                z += u0 + wdiag(code) * (d.rv - masked_stencil(code, u0, nn));
+                z += u0 + wdiag(code) * (d.rv - masked_stencil(code, u0, un));
                 F.t[q] = z;
             }
             zr += static_cast<T>(z) * static_cast<T>(d.r);
@@ -989,12 +1002,11 @@ __global__ void __launch_bounds__(kThreads) mg_net_guess_kernel(const __grid_con
     });
 }
 
-// p' = z + beta p, q = A p'; (p', q) and (p', r). The last block computes alpha = (p', r) / (p', q). z-march: the
-// ring holds p' of every cell.
-template <typename T>
+// p' = z + beta p, q = A p'; (p', q) and (p', r). The last block computes alpha = (p', r) / (p', q). z-march of
+// p'.
+template <typename T, int MR>
 __global__ void __launch_bounds__(kThreads) mg_pq_kernel(const __grid_constant__ MgSolveArgs A) {
     pdl_begin();
-    __shared__ float ring[3][kMPlane];
     const MgLevel& F = A.H.L[0];
     MgState* st = A.st;
     const bool skip = st->fail;  // uniform over the grid
@@ -1006,25 +1018,16 @@ __global__ void __launch_bounds__(kThreads) mg_pq_kernel(const __grid_constant__
         const float* po = A.W.p[par];
         float* pn = A.W.p[par ^ 1];
         const float* r = A.W.r[par];
-        struct Own {
-            uint32_t code;
-            float z, p, r;
-        };
         struct Halo {
             float z, p;
         };
-        march0<false, Own, Halo>(
-            F, A.H.fper, F, ring,
-            [&](bool ok, uint32_t q) {
-                Own d{0u, 0.0f, 0.0f, 0.0f};
-                if (ok) {
-                    d.code = F.code[q];
-                    d.z = Z[q];
-                    d.p = po[q];
-                    d.r = r[q];
-                }
-                return d;
-            },
+        struct None {};
+        struct Own {
+            uint32_t code;
+            float r;
+        };
+        march0<MR, false, Halo, None, Own>(
+            F, A.H.fper, F,
             [&](bool ok, uint32_t q) {
                 Halo d{0.0f, 0.0f};
                 if (ok) {
@@ -1033,12 +1036,17 @@ __global__ void __launch_bounds__(kThreads) mg_pq_kernel(const __grid_constant__
                 }
                 return d;
             },
-            [&](const Own& d) { return d.z + fb * d.p; },
-            [&](const Halo& d) { return d.z + fb * d.p; },
-            [&](bool out, uint32_t q, const Own& d, float um1, float u0, float u1, const float* pl, int s) {
-                if (!out) return 0.0f;
-                const float pnb[6] = {pl[s - 1], pl[s + 1], pl[s - MPX], pl[s + MPX], um1, u1};
-                const float qv = masked_stencil(static_cast<uint16_t>(d.code), u0, pnb);
+            [&](const Halo& d, None&) { return d.z + fb * d.p; },
+            [&](bool ok, uint32_t q) {
+                Own d{0u, 0.0f};
+                if (ok) {
+                    d.code = F.code[q];
+                    d.r = r[q];
+                }
+                return d;
+            },
+            [&](uint32_t q, None, const Own& d, float u0, const float* un) {
+                const float qv = masked_stencil(static_cast<uint16_t>(d.code), u0, un);
                 pn[q] = u0;
                 A.W.q[q] = qv;
                 pq += static_cast<T>(u0) * static_cast<T>(qv);
@@ -1430,17 +1438,28 @@ dim3 wave(K kernel, const MgLevel& L, int depth) {
     return dim3(tx, ty, gz);
 }
 
-// Grid of a level-0 z-march kernel: the same depth codes over its (column, plane pair) units (4 = one unit per
-// block).
-template <class K>
+// Rows of a thread of a level-0 z-march kernel: 4, or 2 where 4 would leave a warp of the chip's one wave without a plane
+// pair of its own.
+constexpr uint32_t kMarchWideCells = 80u * 80u * 80u;
+inline int march_rows(const MgLevel& L) { return L.n >= kMarchWideCells ? 4 : 2; }
+
+// Grid of a level-0 z-march kernel: the same depth codes over its (tile, plane pair) units (4 = one unit per block).
+template <int MR, class K>
 unsigned march_grid(K kernel, const MgLevel& L, int depth) {
-    const long long units = march_units(L).total;
+    const long long units = march_units<MR>(L).total;
     long long blocks = units;
     if (depth < kMgWaveCount - 1) {
         const int resident = resident_blocks(kernel);
         blocks = depth <= 0 ? resident / 2 : static_cast<long long>(resident) << (depth - 1);
     }
     return static_cast<unsigned>(std::max<long long>(1, std::min(blocks, units)));
+}
+// Launches the instance of a z-march kernel that the level's size asks for: k4 and k2 are its instances for MR = 4 and 2.
+template <class K, class... Args>
+void launch_march(K k4, K k2, const MgSolveArgs& A, cudaStream_t s, Args&&... args) {
+    const MgLevel& L = A.H.L[0];
+    if (march_rows(L) == 4) launch_pdl(k4, march_grid<4>(k4, L, A.wave), kThreads, 0, s, A, std::forward<Args>(args)...);
+    else launch_pdl(k2, march_grid<2>(k2, L, A.wave), kThreads, 0, s, A, std::forward<Args>(args)...);
 }
 
 // Adds a `while` node after the capture's current dependencies and captures `body` into it on `body_stream`.
@@ -1475,8 +1494,8 @@ cudaError_t add_while(cudaStream_t s, cudaStream_t body_stream, cudaGraphConditi
 // The level-0 update of the solve's preconditioner kind.
 template <typename T>
 void launch_update(const MgSolveArgs& A, int initial, cudaGraphConditionalHandle h, int in_graph, int net_loop, cudaStream_t s) {
-    if (A.learned) launch_pdl(mg_update_kernel<T, true>, march_grid(mg_update_kernel<T, true>, A.H.L[0], A.wave), kThreads, 0, s, A, initial, h, in_graph, net_loop);
-    else launch_pdl(mg_update_kernel<T, false>, march_grid(mg_update_kernel<T, false>, A.H.L[0], A.wave), kThreads, 0, s, A, initial, h, in_graph, 0);
+    if (A.learned) launch_march(mg_update_kernel<T, true, 4>, mg_update_kernel<T, true, 2>, A, s, initial, h, in_graph, net_loop);
+    else launch_march(mg_update_kernel<T, false, 4>, mg_update_kernel<T, false, 2>, A, s, initial, h, in_graph, 0);
 }
 
 // The V-cycle below level 0: restrictions of levels 1..g-1, the block-level cycle, the up passes of levels g-1..1,
@@ -1506,18 +1525,18 @@ void launch_body(const MgSolveArgs& A, int net, cudaGraphConditionalHandle h, in
     launch_coarse_cycle(A, block_bytes, bs);
     if (net) {  // z = z_V + N(r - A z_V), post-smoothed: the network corrects what the V-cycle leaves
         const LearnedSolve& N = *A.net;
-        launch_pdl(mg_smooth0_kernel<T, false>, march_grid(mg_smooth0_kernel<T, false>, L0, A.wave), kThreads, 0, bs, A);
+        launch_march(mg_smooth0_kernel<T, false, 4>, mg_smooth0_kernel<T, false, 2>, A, bs);
         launch_pdl(mg_net_residual_kernel<T>, wave(mg_net_residual_kernel<T>, L0, A.wave), kBlock, 0, bs, A);
         if (net_forward(N.images, N.acts, A.H.L[1].zp, nullptr, nullptr, &A.st->net_rr, N.occupancy, bs, &A.st->net_off) != cudaSuccess) return;
         launch_pdl(mg_net_prolong_kernel, wave(mg_net_prolong_kernel, A.H.L[1], A.wave), kBlock, 0, bs, A.H, A.st, N.acts.y, &A.st->net_rr, N.fine);
         launch_pdl(mg_net_gamma_kernel<T>, wave(mg_net_gamma_kernel<T>, L0, A.wave), kBlock, 0, bs, A, N.fine);
-        launch_pdl(mg_net_add_kernel<T>, march_grid(mg_net_add_kernel<T>, L0, A.wave), kThreads, 0, bs, A, N.fine);
-        launch_pdl(mg_pq_kernel<T>, march_grid(mg_pq_kernel<T>, L0, A.wave), kThreads, 0, bs, A);
-        launch_pdl(mg_update_kernel<T, true>, march_grid(mg_update_kernel<T, true>, L0, A.wave), kThreads, 0, bs, A, 0, h, in_graph, 1);
+        launch_march(mg_net_add_kernel<T, 4>, mg_net_add_kernel<T, 2>, A, bs, static_cast<const float*>(N.fine));
+        launch_march(mg_pq_kernel<T, 4>, mg_pq_kernel<T, 2>, A, bs);
+        launch_march(mg_update_kernel<T, true, 4>, mg_update_kernel<T, true, 2>, A, bs, 0, h, in_graph, 1);
         return;
     }
-    launch_pdl(mg_smooth0_kernel<T, true>, march_grid(mg_smooth0_kernel<T, true>, L0, A.wave), kThreads, 0, bs, A);
-    launch_pdl(mg_pq_kernel<T>, march_grid(mg_pq_kernel<T>, L0, A.wave), kThreads, 0, bs, A);
+    launch_march(mg_smooth0_kernel<T, true, 4>, mg_smooth0_kernel<T, true, 2>, A, bs);
+    launch_march(mg_pq_kernel<T, 4>, mg_pq_kernel<T, 2>, A, bs);
     launch_update<T>(A, 0, h, in_graph, 0, bs);
 }
 
