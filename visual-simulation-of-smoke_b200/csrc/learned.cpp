@@ -84,8 +84,12 @@ struct SmokeB200Net_t {
     VolumeDims dims{};
     NetActs acts{};
     NetGrads grads{};
+    NetSide side{};
 
     ~SmokeB200Net_t() {
+        if (side.done) cudaEventDestroy(side.done);
+        if (side.ready) cudaEventDestroy(side.ready);
+        if (side.stream) cudaStreamDestroy(side.stream);
         if (work) cudaFree(work);
         if (mem) cudaFree(mem);
     }
@@ -100,6 +104,9 @@ struct SmokeB200Net_t {
         v = reinterpret_cast<float*>(p + 3 * pbytes);
         net_images_bind(images, p + 4 * pbytes);
         check(cudaMemset(mem, 0, 4 * pbytes + net_images_bytes()), "network parameters");
+        check(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking), "network stream");
+        check(cudaEventCreateWithFlags(&side.ready, cudaEventDisableTiming), "network event");
+        check(cudaEventCreateWithFlags(&side.done, cudaEventDisableTiming), "network event");
     }
 
     // Workspace (activations and gradients) for a volume; reallocated when the volume changes size.
@@ -201,7 +208,7 @@ SmokeSimulationResult smoke_b200_net_gradient_cuda(SmokeB200Net net, int nx, int
         check(cudaMemsetAsync(net->acts.error, 0, sizeof(unsigned), s), "network status");
         check(cudaMemsetAsync(net->grads.sums, 0, 2 * sizeof(double), s), "network loss");
         check(net_forward(net->images, net->acts, rhs, nullptr, nullptr, nullptr, occupancy, s), "network forward");
-        check(net_backward(net->images, net->acts, net->grads, nullptr, target, occupancy, net->grad, 0, s), "network backward");
+        check(net_backward(net->images, net->acts, net->grads, nullptr, target, occupancy, net->grad, 0, s, net->side), "network backward");
         net->check_error(s);
         if (grad_out) check(cudaMemcpy(grad_out, net->grad, static_cast<size_t>(kNetParams) * sizeof(float), cudaMemcpyDeviceToHost), "network gradient");
         if (loss_out) check(cudaMemcpy(loss_out, net->grads.sums + 1, sizeof(double), cudaMemcpyDeviceToHost), "network loss");
@@ -219,7 +226,7 @@ SmokeSimulationResult smoke_b200_net_train_cuda(SmokeB200Net net, int nx, int ny
         check(cudaMemsetAsync(net->grads.sums, 0, 2 * sizeof(double), s), "network loss");
         for (uint32_t i = 0; i < count; ++i) {
             check(net_forward(net->images, net->acts, rhs + i * n, nullptr, nullptr, nullptr, occupancy + i * n, s), "network forward");
-            check(net_backward(net->images, net->acts, net->grads, nullptr, target + i * n, occupancy + i * n, net->grad, i > 0 ? 1 : 0, s), "network backward");
+            check(net_backward(net->images, net->acts, net->grads, nullptr, target + i * n, occupancy + i * n, net->grad, i > 0 ? 1 : 0, s, net->side), "network backward");
         }
         net->adam_step += 1;
         check(net_adam(net->params, net->grad, net->m, net->v, learning_rate, net->adam_step, 1.0f / static_cast<float>(count), net->images, s), "adam");

@@ -92,7 +92,6 @@ __global__ void __launch_bounds__(kConvThreads) conv3_kernel(const __grid_consta
     __shared__ uint64_t full[S::kStages], freed[S::kStages], done[2], drained[2], wbar;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    pdl_trigger();
     const int t = threadIdx.x, warp = t >> 5;
     const int chunk = blockIdx.y;
     for (int st = 0; st < S::kStages; ++st)  // the slack after each box stays zero (read by the padding tap, times zero weights)
@@ -116,6 +115,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3_kernel(const __grid_consta
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_trigger();  // after the allocation: a later kernel's block must not take the tensor memory that one of ours still asks for
     pdl_wait();  // the set-up above overlaps the previous kernel's tail
     if (a.skip && *a.skip) {  // uniform: every block reads the same word
         if (warp == 0) tc::tmem_free(tmem, S::kTmemCols);
@@ -303,7 +303,6 @@ __global__ void __launch_bounds__(kConvThreads) conv3_band_kernel(const __grid_c
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     constexpr uint32_t kCols = 32;  // two 16-column accumulators
-    pdl_trigger();
     const int t = threadIdx.x, warp = t >> 5;
     if (t == 0) {
         for (int st = 0; st < kBandStages; ++st) {
@@ -323,6 +322,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3_band_kernel(const __grid_c
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_trigger();  // after the allocation: a later kernel's block must not take the tensor memory that one of ours still asks for
     pdl_wait();  // the set-up above overlaps the previous kernel's tail
     if (a.skip && *a.skip) {  // uniform: every block reads the same word
         if (warp == 0) tc::tmem_free(tmem, kCols);
@@ -628,6 +628,8 @@ __global__ void __launch_bounds__(kEpiThreads) wgrad_kernel(const __grid_constan
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    pdl_trigger();  // after the allocation: a later kernel's block must not take the tensor memory that one of ours still asks for
+    pdl_wait();  // the set-up above overlaps the previous kernel's tail
     constexpr uint32_t idesc = tc::idesc_bf16_f32(128, GN, true, true);
     const uint32_t a_base = tc::smem_addr(As), b_base = tc::smem_addr(Bs);
     const uint32_t chunks = (a.n + kWgradCells - 1) / kWgradCells;
@@ -711,8 +713,11 @@ __global__ void __launch_bounds__(kEpiThreads) wgrad_kernel(const __grid_constan
 }
 
 // grad[w(tap, ci, co)] (+)= sum over blocks of partial[b][tap * cs + ci][co]; grad[bias co] likewise from row
-// 27 * cs.
+// 27 * cs. The sum runs over the blocks in order, eight loads in flight at a time (one by one, each waited for L2: 11 us a
+// layer on a 32^3 sample, now 4).
 __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int blocks, int m_pad, int gn, int cs, int cin, int cout, int accumulate, float* __restrict__ grad) {
+    pdl_trigger();
+    pdl_wait();
     const int wcount = 27 * cin * cout;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < wcount + cout; i += gridDim.x * blockDim.x) {
         int row, co;
@@ -724,8 +729,18 @@ __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int block
             co = i - wcount;
             row = 27 * cs;
         }
+        const size_t pitch = static_cast<size_t>(m_pad) * gn;
+        const float* p = partial + static_cast<size_t>(row) * gn + co;
         float sum = 0.0f;
-        for (int b = 0; b < blocks; ++b) sum += partial[(static_cast<size_t>(b) * m_pad + row) * gn + co];
+        int b = 0;
+        for (; b + 8 <= blocks; b += 8, p += 8 * pitch) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = p[k * pitch];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sum += v[k];
+        }
+        for (; b < blocks; ++b, p += pitch) sum += *p;
         grad[i] = accumulate ? grad[i] + sum : sum;
     }
 }
@@ -750,6 +765,8 @@ __device__ __forceinline__ uint32_t cell_at(const VolumeDims& d, int x, int y, i
 
 // sum of squares into *out (FP64)
 __global__ void sumsq_kernel(const float* __restrict__ v, uint32_t n, double* __restrict__ out) {
+    pdl_trigger();
+    pdl_wait();
     double s = 0.0;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) s += static_cast<double>(v[q]) * v[q];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -832,6 +849,8 @@ __global__ void up_add_kernel(VolumeDims f, VolumeDims c, const __nv_bfloat16* _
 // Backward of up (sum over the children), then the ReLU gate of the coarse activation: dc[Q] = (sum df[q]) * [act > 0]
 template <int C>
 __global__ void up_bwd_relu_kernel(VolumeDims f, VolumeDims c, const __nv_bfloat16* __restrict__ dfine, const __nv_bfloat16* __restrict__ act, __nv_bfloat16* __restrict__ dcoarse) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int G = C / 8;
     const uint64_t items = static_cast<uint64_t>(c.n) * G;
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < items; i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
@@ -862,6 +881,8 @@ __global__ void up_bwd_relu_kernel(VolumeDims f, VolumeDims c, const __nv_bfloat
 // gate of the fine activation: df[q] = (skip[q] + dc[parent] / count) * [act > 0]
 template <int C>
 __global__ void pool_bwd_add_relu_kernel(VolumeDims f, VolumeDims c, const __nv_bfloat16* __restrict__ skip, const __nv_bfloat16* __restrict__ dcoarse, const __nv_bfloat16* __restrict__ act, __nv_bfloat16* __restrict__ dfine) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int G = C / 8;
     const uint64_t items = static_cast<uint64_t>(f.n) * G;
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < items; i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
@@ -893,6 +914,8 @@ __global__ void net_output_kernel(VolumeDims d, const float* __restrict__ y, con
 // Loss of one sample: L = sum_fluid (y - s t)^2 / sum_fluid (s t)^2 (s the input scale); dy = dL/dy into channel 0 of
 // gy ([n][16] BF16, the other channels 0), L added into *loss. tt = sum_fluid t^2 (from sumsq of the masked target).
 __global__ void net_loss_kernel(VolumeDims d, const float* __restrict__ y, const float* __restrict__ target, const uint8_t* __restrict__ occ, const double* __restrict__ norm2, const double* __restrict__ tt, __nv_bfloat16* __restrict__ gy, double* __restrict__ loss) {
+    pdl_trigger();
+    pdl_wait();
     const double nn = *norm2;
     const double s = nn > 0.0 ? sqrt(static_cast<double>(d.n) / nn) : 0.0;
     const double denom = s * s * *tt;
@@ -913,6 +936,8 @@ __global__ void net_loss_kernel(VolumeDims d, const float* __restrict__ y, const
 
 // masked copy for the target norm: out[q] = fluid ? t[q] : 0
 __global__ void mask_fluid_kernel(uint32_t n, const float* __restrict__ t, const uint8_t* __restrict__ occ, float* __restrict__ out) {
+    pdl_trigger();
+    pdl_wait();
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) out[q] = occ[q] == 0 ? t[q] : 0.0f;
 }
 
@@ -1039,7 +1064,7 @@ cudaError_t layer_wgrad(int L, const VolumeDims& d, const __nv_bfloat16* in, con
         default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    wgrad_reduce_kernel<<<64, 256, 0, s>>>(G.partial, bx, wgrad_mpad(cs), gn, cs, kNet[L].cin, kNet[L].cout, accumulate, grad + net_param_offset(L));
+    launch_pdl(wgrad_reduce_kernel, dim3(glue_blocks(static_cast<uint64_t>(net_param_count(L)))), dim3(kGlueThreads), 0, s, static_cast<const float*>(G.partial), bx, wgrad_mpad(cs), gn, cs, kNet[L].cin, kNet[L].cout, accumulate, grad + net_param_offset(L));
     return cudaGetLastError();
 }
 
@@ -1195,7 +1220,7 @@ cudaError_t net_forward(const NetImages& I, const NetActs& A, const float* r0, c
     cudaError_t e;
     if (norm2 == nullptr) {
         if ((e = cudaMemsetAsync(A.norm2, 0, sizeof(double), s)) != cudaSuccess) return e;
-        sumsq_kernel<<<glue_blocks(d[0].n), kGlueThreads, 0, s>>>(r0, d[0].n, A.norm2);
+        launch_pdl(sumsq_kernel, dim3(glue_blocks(d[0].n)), dim3(kGlueThreads), 0, s, r0, d[0].n, A.norm2);
         norm2 = A.norm2;
     }
     launch_pdl(net_input_kernel, dim3(glue_blocks(d[0].n)), dim3(kGlueThreads), 0, s, d[0], r0, r1, parity, norm2, occ, A.x0, skip);
@@ -1223,44 +1248,54 @@ cudaError_t net_output(const NetActs& A, const double* norm2, const uint8_t* occ
     return cudaGetLastError();
 }
 
-cudaError_t net_backward(const NetImages& I, const NetActs& A, const NetGrads& G, const double* norm2, const float* target, const uint8_t* occ, float* grad, int accumulate, cudaStream_t s) {
+cudaError_t net_backward(const NetImages& I, const NetActs& A, const NetGrads& G, const double* norm2, const float* target, const uint8_t* occ, float* grad, int accumulate, cudaStream_t s, const NetSide& side) {
     const VolumeDims* d = A.d;
     if (norm2 == nullptr) norm2 = A.norm2;
     cudaError_t e = cudaMemsetAsync(G.sums, 0, sizeof(double), s);  // target norm^2 (the loss accumulates)
     if (e != cudaSuccess) return e;
-    mask_fluid_kernel<<<glue_blocks(d[0].n), kGlueThreads, 0, s>>>(d[0].n, target, occ, G.tmask);
-    sumsq_kernel<<<glue_blocks(d[0].n), kGlueThreads, 0, s>>>(G.tmask, d[0].n, G.sums);
-    net_loss_kernel<<<glue_blocks(d[0].n), kGlueThreads, 0, s>>>(d[0], A.y, target, occ, norm2, G.sums, G.gy, G.sums + 1);
+    const dim3 cells(glue_blocks(d[0].n)), threads(kGlueThreads);
+    launch_pdl(mask_fluid_kernel, cells, threads, 0, s, d[0].n, target, occ, G.tmask);
+    launch_pdl(sumsq_kernel, cells, threads, 0, s, static_cast<const float*>(G.tmask), d[0].n, G.sums);
+    launch_pdl(net_loss_kernel, cells, threads, 0, s, d[0], static_cast<const float*>(A.y), target, occ, norm2, static_cast<const double*>(G.sums), G.gy, G.sums + 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    // The weight gradients feed nothing in the chain below, so they run on the side stream as soon as their layer's
+    // gradient exists: the coarse levels' kernels leave most SMs idle.
+    auto wgrad = [&](int L, const VolumeDims& dims, const __nv_bfloat16* in, const __nv_bfloat16* g) {
+        cudaError_t r = cudaEventRecord(side.ready, s);
+        if (r == cudaSuccess) r = cudaStreamWaitEvent(side.stream, side.ready, 0);
+        return r == cudaSuccess ? layer_wgrad(L, dims, in, g, G, grad, accumulate, A.error, side.stream) : r;
+    };
     // g: y = conv_g(s0); s0 = up(u1) + e0
-    if ((e = layer_wgrad(7, d[0], A.s0, G.gy, G, grad, accumulate, A.error, s)) != cudaSuccess) return e;
+    if ((e = wgrad(7, d[0], A.s0, G.gy)) != cudaSuccess) return e;
     if ((e = conv_layer_bwd(7, d[0], I, G.gy, nullptr, G.gs0, A.error, s)) != cudaSuccess) return e;
     // f: u1 = relu(conv_f(s1)); s1 = up(u2) + e1
-    up_bwd_relu_kernel<16><<<glue_blocks_c(d[1].n, 16), kGlueThreads, 0, s>>>(d[0], d[1], G.gs0, A.u1, G.gu1);
-    if ((e = layer_wgrad(6, d[1], A.s1, G.gu1, G, grad, accumulate, A.error, s)) != cudaSuccess) return e;
+    launch_pdl(up_bwd_relu_kernel<16>, dim3(glue_blocks_c(d[1].n, 16)), threads, 0, s, d[0], d[1], static_cast<const __nv_bfloat16*>(G.gs0), static_cast<const __nv_bfloat16*>(A.u1), G.gu1);
+    if ((e = wgrad(6, d[1], A.s1, G.gu1)) != cudaSuccess) return e;
     if ((e = conv_layer_bwd(6, d[1], I, G.gu1, nullptr, G.gs1, A.error, s)) != cudaSuccess) return e;
     // e: u2 = relu(conv_e(s2)); s2 = up(m3) + e2
-    up_bwd_relu_kernel<32><<<glue_blocks_c(d[2].n, 32), kGlueThreads, 0, s>>>(d[1], d[2], G.gs1, A.u2, G.gu2);
-    if ((e = layer_wgrad(5, d[2], A.s2, G.gu2, G, grad, accumulate, A.error, s)) != cudaSuccess) return e;
+    launch_pdl(up_bwd_relu_kernel<32>, dim3(glue_blocks_c(d[2].n, 32)), threads, 0, s, d[1], d[2], static_cast<const __nv_bfloat16*>(G.gs1), static_cast<const __nv_bfloat16*>(A.u2), G.gu2);
+    if ((e = wgrad(5, d[2], A.s2, G.gu2)) != cudaSuccess) return e;
     if ((e = conv_layer_bwd(5, d[2], I, G.gu2, nullptr, G.gs2, A.error, s)) != cudaSuccess) return e;
     // m: m3 = relu(conv_m(e3)); e3 = relu(conv_d(p3)) feeds m only, so its ReLU gate goes into m's backward
-    up_bwd_relu_kernel<64><<<glue_blocks_c(d[3].n, 64), kGlueThreads, 0, s>>>(d[2], d[3], G.gs2, A.m3, G.gm3);
-    if ((e = layer_wgrad(4, d[3], A.e3, G.gm3, G, grad, accumulate, A.error, s)) != cudaSuccess) return e;
+    launch_pdl(up_bwd_relu_kernel<64>, dim3(glue_blocks_c(d[3].n, 64)), threads, 0, s, d[2], d[3], static_cast<const __nv_bfloat16*>(G.gs2), static_cast<const __nv_bfloat16*>(A.m3), G.gm3);
+    if ((e = wgrad(4, d[3], A.e3, G.gm3)) != cudaSuccess) return e;
     if ((e = conv_layer_bwd(4, d[3], I, G.gm3, A.e3, G.ge3, A.error, s)) != cudaSuccess) return e;
     // d: e3 = relu(conv_d(p3)); p3 = pool(e2)
-    if ((e = layer_wgrad(3, d[3], A.p3, G.ge3, G, grad, accumulate, A.error, s)) != cudaSuccess) return e;
+    if ((e = wgrad(3, d[3], A.p3, G.ge3)) != cudaSuccess) return e;
     if ((e = conv_layer_bwd(3, d[3], I, G.ge3, nullptr, G.gp3, A.error, s)) != cudaSuccess) return e;
     // c: e2 = relu(conv_c(p2)) feeds p3 and s2
-    pool_bwd_add_relu_kernel<64><<<glue_blocks_c(d[2].n, 64), kGlueThreads, 0, s>>>(d[2], d[3], G.gs2, G.gp3, A.e2, G.ge2);
-    if ((e = layer_wgrad(2, d[2], A.p2, G.ge2, G, grad, accumulate, A.error, s)) != cudaSuccess) return e;
+    launch_pdl(pool_bwd_add_relu_kernel<64>, dim3(glue_blocks_c(d[2].n, 64)), threads, 0, s, d[2], d[3], static_cast<const __nv_bfloat16*>(G.gs2), static_cast<const __nv_bfloat16*>(G.gp3), static_cast<const __nv_bfloat16*>(A.e2), G.ge2);
+    if ((e = wgrad(2, d[2], A.p2, G.ge2)) != cudaSuccess) return e;
     if ((e = conv_layer_bwd(2, d[2], I, G.ge2, nullptr, G.gp2, A.error, s)) != cudaSuccess) return e;
     // b: e1 = relu(conv_b(p1)) feeds p2 and s1
-    pool_bwd_add_relu_kernel<32><<<glue_blocks_c(d[1].n, 32), kGlueThreads, 0, s>>>(d[1], d[2], G.gs1, G.gp2, A.e1, G.ge1);
-    if ((e = layer_wgrad(1, d[1], A.p1, G.ge1, G, grad, accumulate, A.error, s)) != cudaSuccess) return e;
+    launch_pdl(pool_bwd_add_relu_kernel<32>, dim3(glue_blocks_c(d[1].n, 32)), threads, 0, s, d[1], d[2], static_cast<const __nv_bfloat16*>(G.gs1), static_cast<const __nv_bfloat16*>(G.gp2), static_cast<const __nv_bfloat16*>(A.e1), G.ge1);
+    if ((e = wgrad(1, d[1], A.p1, G.ge1)) != cudaSuccess) return e;
     if ((e = conv_layer_bwd(1, d[1], I, G.ge1, nullptr, G.gp1, A.error, s)) != cudaSuccess) return e;
     // a: e0 = relu(conv_a(x0)) feeds p1 and s0
-    pool_bwd_add_relu_kernel<16><<<glue_blocks_c(d[0].n, 16), kGlueThreads, 0, s>>>(d[0], d[1], G.gs0, G.gp1, A.e0, G.ge0);
-    return layer_wgrad(0, d[0], A.x0, G.ge0, G, grad, accumulate, A.error, s);
+    launch_pdl(pool_bwd_add_relu_kernel<16>, dim3(glue_blocks_c(d[0].n, 16)), threads, 0, s, d[0], d[1], static_cast<const __nv_bfloat16*>(G.gs0), static_cast<const __nv_bfloat16*>(G.gp1), static_cast<const __nv_bfloat16*>(A.e0), G.ge0);
+    if ((e = wgrad(0, d[0], A.x0, G.ge0)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(side.done, side.stream)) != cudaSuccess) return e;
+    return cudaStreamWaitEvent(s, side.done, 0);
 }
 
 cudaError_t net_adam(float* w, const float* grad, float* m, float* v, float lr, int step, float gscale, const NetImages& I, cudaStream_t s) {

@@ -126,9 +126,16 @@ void net_grads_bind(NetGrads& G, void* base, const VolumeDims& d0);
 cudaError_t net_forward(const NetImages& I, const NetActs& A, const float* r0, const float* r1, const int* parity, const double* norm2, const uint8_t* occ, cudaStream_t s, const uint32_t* skip = nullptr);
 // out = fluid ? A.y / s : 0 (the preconditioned vector with the input's scale restored).
 cudaError_t net_output(const NetActs& A, const double* norm2, const uint8_t* occ, float* out, cudaStream_t s);
+// Second stream of a backward pass with its two events: `ready` marks a layer's gradient on the caller's stream, `done` the
+// last weight gradient on this one.
+struct NetSide {
+    cudaStream_t stream;
+    cudaEvent_t ready, done;
+};
 // Loss of the last forward pass against `target` and the parameter gradient: grad (kNetParams floats) is
-// overwritten, or accumulated into when `accumulate`; the loss is added into G.sums[1].
-cudaError_t net_backward(const NetImages& I, const NetActs& A, const NetGrads& G, const double* norm2, const float* target, const uint8_t* occ, float* grad, int accumulate, cudaStream_t s);
+// overwritten, or accumulated into when `accumulate`; the loss is added into G.sums[1]. Everything is
+// ordered on `s`: the weight gradients run on side.stream, which `s` waits for at the end.
+cudaError_t net_backward(const NetImages& I, const NetActs& A, const NetGrads& G, const double* norm2, const float* target, const uint8_t* occ, float* grad, int accumulate, cudaStream_t s, const NetSide& side);
 // One Adam step on w with moments m, v (step >= 1), gradient scaled by gscale; then the images are repacked.
 cudaError_t net_adam(float* w, const float* grad, float* m, float* v, float lr, int step, float gscale, const NetImages& I, cudaStream_t s);
 
