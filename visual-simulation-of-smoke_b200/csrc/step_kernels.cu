@@ -617,47 +617,94 @@ __global__ void __launch_bounds__(kThreads) stencil_code_kernel(const __grid_con
     codes[q] = static_cast<uint16_t>(mask | (diag << 8) | kCodeActive);
 }
 
-// Nearest-fluid source of each solid cell (:1243-1290): first Chebyshev shell (radius 1, 2, ...) holding a fluid
-// cell, smallest squared distance in it, first in (dz, dy, dx) scan order on ties, density periodicity. Only the
-// shell surface is enumerated, in the same order as a full-cube scan.
-__global__ void __launch_bounds__(kThreads) fill_build_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor_ptr, FillEntry* __restrict__ list, uint32_t* __restrict__ count) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= P.n || occ[q] == 0) return;
-    int32_t best = -1;
-    if (*anchor_ptr < static_cast<int32_t>(P.n)) {  // at least one fluid cell exists
+// The solid cells, in no particular order, each without a source (a warp's cells take one slot range).
+__global__ void __launch_bounds__(kThreads) fill_list_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, FillEntry* __restrict__ list, uint32_t* __restrict__ count) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const bool solid = q < P.n && occ[q] != 0;
+    const uint32_t solids = __ballot_sync(0xffffffffu, solid);
+    if (solids == 0) return;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, static_cast<uint32_t>(__popc(solids)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (solid) list[base + __popc(solids & ((1u << lane) - 1u))] = FillEntry{q, -1};
+}
+
+// Cell i of the surface of the cube of radius r (24 r^2 + 2 of them): the two z faces, then the rings between them.
+__device__ __forceinline__ void shell_offset(uint32_t i, int r, int& dx, int& dy, int& dz) {
+    const uint32_t side = 2u * r + 1u, face = side * side;
+    if (i < 2u * face) {
+        const uint32_t k = i < face ? i : i - face, row = k / side;
+        dz = i < face ? -r : r;
+        dy = static_cast<int>(row) - r;
+        dx = static_cast<int>(k - row * side) - r;
+        return;
+    }
+    i -= 2u * face;
+    const uint32_t ring = 8u * r, layer = i / ring;
+    uint32_t k = i - layer * ring;
+    dz = static_cast<int>(layer) - r + 1;
+    if (k < 2u * side) {
+        dy = k < side ? -r : r;
+        dx = static_cast<int>(k < side ? k : k - side) - r;
+    } else {
+        k -= 2u * side;
+        dy = static_cast<int>(k >> 1) - r + 1;
+        dx = (k & 1u) ? r : -r;
+    }
+}
+
+// Nearest-fluid source of each solid cell (:1243-1290): first Chebyshev shell (radius 1, 2, ...) holding a fluid cell,
+// smallest squared distance in it, first in (dz, dy, dx) scan order on ties, density periodicity. A cell at depth r has
+// (2 r + 1)^3 neighbours to look at, one load latency after the other if a thread walks them, and the deepest cell decides
+// the time; so a warp takes a cell and its lanes share each shell. The scan order is part of the key that the lanes reduce.
+// A sphere of solid cells in 96 x 128 x 96: 452 us with a thread per cell, 42 with these two kernels.
+__global__ void __launch_bounds__(kThreads) fill_source_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor_ptr, FillEntry* __restrict__ list, const uint32_t* __restrict__ count) {
+    if (*anchor_ptr >= static_cast<int32_t>(P.n)) return;  // no fluid cell exists
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kThreads / 32), entries = *count;
+    const int max_radius = imax(P.nx, imax(P.ny, P.nz));
+    for (uint32_t e = blockIdx.x * (kThreads / 32) + threadIdx.x / 32; e < entries; e += warps) {
         int x, y, z;
-        cell_xyz(P, q, x, y, z);
-        const int max_radius = imax(P.nx, imax(P.ny, P.nz));
+        cell_xyz(P, list[e].cell, x, y, z);
+        int32_t best = -1;
         for (int r = 1; r <= max_radius && best < 0; ++r) {
+            const uint64_t cells = 24ull * r * r + 2ull;
             int best_d2 = 0x7fffffff;
-            for (int dz = -r; dz <= r; ++dz) {
-                for (int dy = -r; dy <= r; ++dy) {
-                    const bool full_row = (dz == -r || dz == r || dy == -r || dy == r);
-                    const int step = full_row ? 1 : 2 * r;
-                    for (int dx = -r; dx <= r; dx += step) {
-                        int c[3] = {x + dx, y + dy, z + dz};
-                        const int nn[3] = {P.nx, P.ny, P.nz};
-                        bool ok = true;
+            uint64_t best_order = ~0ull;
+            for (uint64_t i = lane; i < cells; i += 32u) {
+                int dx, dy, dz;
+                shell_offset(static_cast<uint32_t>(i), r, dx, dy, dz);
+                int c[3] = {x + dx, y + dy, z + dz};
+                const int nn[3] = {P.nx, P.ny, P.nz};
+                bool ok = true;
 #pragma unroll
-                        for (int a = 0; a < 3; ++a) {
-                            if (P.dper[a]) c[a] = wrapi(c[a], nn[a]);
-                            ok = ok && c[a] >= 0 && c[a] < nn[a];
-                        }
-                        if (!ok) continue;
-                        const uint32_t nb = cidx(P, c[0], c[1], c[2]);
-                        if (occ[nb] != 0) continue;
-                        const int d2 = dx * dx + dy * dy + dz * dz;
-                        if (d2 < best_d2) {
-                            best_d2 = d2;
-                            best = static_cast<int32_t>(nb);
-                        }
-                    }
+                for (int a = 0; a < 3; ++a) {
+                    if (P.dper[a]) c[a] = wrapi(c[a], nn[a]);
+                    ok = ok && c[a] >= 0 && c[a] < nn[a];
+                }
+                if (!ok) continue;
+                const uint32_t nb = cidx(P, c[0], c[1], c[2]);
+                if (occ[nb] != 0) continue;
+                const int d2 = dx * dx + dy * dy + dz * dz;
+                const uint64_t order = (static_cast<uint64_t>(dz + r) << 42) | (static_cast<uint64_t>(dy + r) << 21) | static_cast<uint64_t>(dx + r);
+                if (d2 < best_d2 || (d2 == best_d2 && order < best_order)) {
+                    best_d2 = d2;
+                    best_order = order;
+                    best = static_cast<int32_t>(nb);
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                const int d2 = __shfl_xor_sync(0xffffffffu, best_d2, o);
+                const uint64_t order = __shfl_xor_sync(0xffffffffu, best_order, o);
+                const int32_t cell = __shfl_xor_sync(0xffffffffu, best, o);
+                if (d2 < best_d2 || (d2 == best_d2 && order < best_order)) {
+                    best_d2 = d2;
+                    best_order = order;
+                    best = cell;
                 }
             }
         }
+        if (lane == 0) list[e].source = best;
     }
-    const uint32_t slot = atomicAdd(count, 1u);
-    list[slot] = FillEntry{q, best};
 }
 
 __global__ void fill_value_kernel(float* __restrict__ dst, float value, uint64_t count) {
@@ -848,7 +895,10 @@ cudaError_t launch_stencil_codes(const StepParams& P, const uint8_t* occ, const 
 cudaError_t launch_fill_build(const StepParams& P, const uint8_t* occ, const int32_t* anchor, FillEntry* list, uint32_t* count, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    fill_build_kernel<<<blocks_for(P.n), kThreads, 0, s>>>(P, occ, anchor, list, count);
+    fill_list_kernel<<<blocks_for(P.n), kThreads, 0, s>>>(P, occ, list, count);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    constexpr unsigned kFillBlocks = 148 * 8;  // one resident wave; the entry count is on the device
+    fill_source_kernel<<<std::min(kFillBlocks, blocks_for(P.n)), kThreads, 0, s>>>(P, occ, anchor, list, count);
     return cudaGetLastError();
 }
 
