@@ -179,21 +179,23 @@ __global__ void __launch_bounds__(kConvThreads) conv3_kernel(const __grid_consta
                     weights_ready = true;
                 }
                 tc::fence_after_sync();
-                const uint32_t a_base = tc::smem_addr(smem + st * S::kStage);
-#pragma unroll 1
+                // Unrolled, so that each MMA's descriptors are its group's plus a constant (16-byte units of the address field).
+                const uint64_t a_desc = tc::smem_desc(tc::smem_addr(smem + st * S::kStage), 0u, kRow);
+                const uint64_t b_desc = tc::smem_desc(b_base + static_cast<uint32_t>(g) * (NC / 8) * 256u, (NC / 8) * 128u, 128u);
+#pragma unroll
                 for (int k = 0; k < S::kMmas; ++k) {
                     uint32_t start, lbo, k0;
                     if constexpr (CS == 8) {  // taps 2k and 2k + 1 (tap 27: zero weights, any finite A)
-                        start = a_base + tap_offset(2 * k);
+                        start = tap_offset(2 * k);
                         lbo = 2 * k + 1 < 27 ? tap_offset(2 * k + 1) - tap_offset(2 * k) : 16u;
                         k0 = 16u * k;
                     } else {  // tap k, channel planes 2g and 2g + 1
-                        start = a_base + tap_offset(k);
+                        start = tap_offset(k);
                         lbo = kPlane;
-                        k0 = static_cast<uint32_t>(k * CS + 16 * g);
+                        k0 = static_cast<uint32_t>(k * CS);
                     }
-                    const uint64_t bd = tc::smem_desc(b_base + (k0 / 8u) * (NC / 8) * 128u, (NC / 8) * 128u, 128u);
-                    tc::mma_bf16(tmem + static_cast<uint32_t>(b * NC), tc::smem_desc(start, lbo, kRow), bd, idesc, (g > 0 || k > 0) ? 1u : 0u);
+                    const uint64_t ad = a_desc + (static_cast<uint64_t>(lbo / 16u) << 16) + start / 16u, bd = b_desc + (k0 / 8u) * (NC / 8) * 8u;
+                    tc::mma_bf16(tmem + static_cast<uint32_t>(b * NC), ad, bd, idesc, (g > 0 || k > 0) ? 1u : 0u);
                 }
                 tc::commit(&freed[st]);
                 if (g == S::kGroups - 1) tc::commit(&done[b]);
@@ -380,13 +382,11 @@ __global__ void __launch_bounds__(kConvThreads) conv3_band_kernel(const __grid_c
                     weights_ready = true;
                 }
                 tc::fence_after_sync();
-                const uint32_t a_base = tc::smem_addr(smem + st * kBandStage);
-#pragma unroll 1
-                for (int k = 0; k < 27; ++k) {  // box plane zz = k / 9 (input plane j = 3 box + zz), in-plane tap k % 9
-                    const int j = 3 * box + k / 9, tap = k % 9;
-                    const uint64_t bd = tc::smem_desc(b_base + static_cast<uint32_t>(tap) * kBandTap + static_cast<uint32_t>(kBandJ - 1 - j) * 16u, kBandBlock, 128u);
-                    tc::mma_bf16(tmem + static_cast<uint32_t>(b * 16), tc::smem_desc(a_base + tap_offset(k), kPlane, kRow), bd, idesc, (box > 0 || k > 0) ? 1u : 0u);
-                }
+                const uint64_t a_desc = tc::smem_desc(tc::smem_addr(smem + st * kBandStage), kPlane, kRow);
+                const uint64_t b_desc = tc::smem_desc(b_base + static_cast<uint32_t>(kBandJ - 1 - 3 * box) * 16u, kBandBlock, 128u);
+#pragma unroll
+                for (int k = 0; k < 27; ++k)  // box plane zz = k / 9 (input plane j = 3 box + zz), in-plane tap k % 9
+                    tc::mma_bf16(tmem + static_cast<uint32_t>(b * 16), a_desc + tap_offset(k) / 16u, b_desc + static_cast<uint64_t>((k % 9) * (kBandTap / 16u)) - static_cast<uint64_t>(k / 9), idesc, (box > 0 || k > 0) ? 1u : 0u);
                 tc::commit(&freed[st]);
                 if (box == kBandItems - 1) tc::commit(&done[b]);
                 issued = i + 1;
@@ -666,14 +666,14 @@ __global__ void __launch_bounds__(kEpiThreads) wgrad_kernel(const __grid_constan
         __syncthreads();
         tc::fence_after_sync();
         if (t == 0) {
-#pragma unroll 1
-            for (int mt = 0; mt < m_tiles; ++mt)
-#pragma unroll 1
-                for (int k = 0; k < kWgradCells / 16; ++k) {
-                    // K step k: cell groups 2k, 2k + 1 (LBO: next cell group); SBO: next 8 rows of M (or N)
-                    const uint64_t ad = tc::smem_desc(a_base + (2 * k * S::kMGroups + mt * 16) * 128u, S::kMGroups * 128u, 128u);
-                    const uint64_t bd = tc::smem_desc(b_base + (2 * k * (GN / 8)) * 128u, (GN / 8) * 128u, 128u);
-                    tc::mma_bf16(tmem + static_cast<uint32_t>(mt * GN), ad, bd, idesc, (any || k > 0) ? 1u : 0u);
+            // K step k: cell groups 2k, 2k + 1 (LBO: next cell group); SBO: next 8 rows of M (or N)
+            const uint64_t a_desc = tc::smem_desc(a_base, S::kMGroups * 128u, 128u), b_desc = tc::smem_desc(b_base, (GN / 8) * 128u, 128u);
+#pragma unroll
+            for (int mt = 0; mt < S::kMT; ++mt)
+                if (mt < m_tiles) {
+#pragma unroll
+                    for (int k = 0; k < kWgradCells / 16; ++k)
+                        tc::mma_bf16(tmem + static_cast<uint32_t>(mt * GN), a_desc + (2 * k * S::kMGroups + mt * 16) * 8u, b_desc + (2 * k * (GN / 8)) * 8u, idesc, (any || k > 0) ? 1u : 0u);
                 }
             tc::commit(&bar);
         }
