@@ -194,6 +194,9 @@ struct SmokeSimulationContext_t {
             if (mg.L[l].n > kMgBlockLevelCells || block_words * 4u > kMgBlockBytes) break;
             mg.grid_levels = l;
         }
+        mg.block_cells = 0;
+        for (int l = mg.grid_levels; l < mg.levels; ++l) mg.block_cells += mg.L[l].n;
+        slots.push_back({reinterpret_cast<void**>(&mg.block_table), mg.block_cells * sizeof(BlockCell)});
         auto align = [](size_t v) { return (v + 255) & ~size_t(255); };
         size_t total = 0;
         for (const Slot& s : slots) total += align(s.bytes);

@@ -169,8 +169,8 @@ struct PcgLaunchShape {
 // 7-point stencil of its fluid cells (the fine rules without the anchor).
 constexpr int kMgMaxLevels = 12;
 constexpr uint32_t kMgBlockLevelCells = 512;   // levels this small may run inside one block, in shared memory
-constexpr uint32_t kMgBlockBytes = 16 * 1024;  // shared memory for those levels (3 floats + 1 code per cell)
-// Shared-memory words of one block-level level of n cells: r, zp, t and the 16-bit codes (padded pairs).
+constexpr uint32_t kMgBlockBytes = 16 * 1024;  // limit of those levels' arrays (3 floats + 1 code per cell)
+// Words of a level of n cells that the limit above counts: r, zp, t and the 16-bit codes (padded pairs).
 __host__ __device__ constexpr uint32_t mg_block_words(uint32_t n) { return 3u * n + (n + 2u) / 2u; }
 // Bit of the operator code that marks a cell whose unknown is solved for (fluid; at level 0 also not the anchor).
 constexpr uint16_t kCodeActive = 1u << 12;
@@ -184,11 +184,19 @@ struct MgLevel {
     float* zp;        // correction (level 0: the preconditioned residual z)
     float* t;         // scratch of the level
 };
+// What a block level's cell takes from the grid and its codes alone; cells of all block levels are numbered through.
+struct BlockCell {
+    uint4 nbr;       // 16 bits each: the 6 stencil neighbours, then the operator code
+    uint4 corners;   // the 8 corners of the prolongation onto the cell: cells of the next level, 0xffff for minus the parent
+    uint4 children;  // the 8 children on the level before, 0xffff for one that does not exist
+};
 struct MgHierarchy {
     int levels;       // >= 2
     int grid_levels;  // levels [0, grid_levels) run on the whole grid; coarser ones inside block 0's shared memory
     int fper[3];
     int fout[6];      // non-periodic OUTFLOW faces (x-, x+, y-, y+, z-, z+): prolongation extrapolates to -parent there
+    uint32_t block_cells;    // cells of the levels from grid_levels on
+    BlockCell* block_table;  // their entries
     MgLevel L[kMgMaxLevels];
 };
 // Level-0 vectors of the multigrid FCG solve (the residual and search direction are double-buffered: a pass reads
