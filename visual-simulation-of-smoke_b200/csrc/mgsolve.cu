@@ -1156,9 +1156,9 @@ __device__ __forceinline__ uint4 block_corners(const MgLevel& C, uint32_t base, 
     return pack_halves(idx);
 }
 
-// The table entries of every block level's cells.
-__global__ void __launch_bounds__(kThreads) mg_block_table_kernel(const __grid_constant__ MgHierarchy H) {
-    uint32_t base = 0, fine = 0, q = blockIdx.x * kThreads + threadIdx.x;
+// Table entry of cell q of the block levels.
+__device__ void block_table_entry(const MgHierarchy& H, uint32_t q) {
+    uint32_t base = 0, fine = 0;
     int l = H.grid_levels;
     for (; l < H.levels && q >= H.L[l].n; ++l) {
         fine = base;
@@ -1748,14 +1748,15 @@ cudaError_t run_typed(const MgSolveArgs& A, PcgStatusDevice* out, cudaStream_t s
 }
 
 // ---------------------------------------------------------------------------------------------- hierarchy setup
-__global__ void mg_fluid0_kernel(uint32_t n, const uint8_t* __restrict__ occ, uint8_t* __restrict__ fluid) {
+// Fluid marks of level 0, and zeroes in the two spare entries past its codes.
+__global__ void mg_fluid0_kernel(uint32_t n, const uint8_t* __restrict__ occ, uint8_t* __restrict__ fluid, uint16_t* __restrict__ code) {
+    pdl_begin();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n) fluid[q] = occ[q] == 0 ? 1 : 0;
+    if (q < 2u) code[n + q] = 0;
 }
 
-__global__ void mg_coarsen_kernel(const MgLevel F, const MgLevel C) {
-    const uint32_t cq = blockIdx.x * blockDim.x + threadIdx.x;
-    if (cq >= C.n) return;
+__device__ void coarsen_cell(const MgLevel& F, const MgLevel& C, uint32_t cq) {
     int X, Y, Z;
     lxyz(C, cq, X, Y, Z);
     uint8_t any = 0;
@@ -1767,11 +1768,15 @@ __global__ void mg_coarsen_kernel(const MgLevel F, const MgLevel C) {
             }
     C.fluid[cq] = any;
 }
+__global__ void mg_coarsen_kernel(const MgLevel F, const MgLevel C) {
+    pdl_begin();
+    const uint32_t cq = blockIdx.x * blockDim.x + threadIdx.x;
+    if (cq < C.n) coarsen_cell(F, C, cq);
+}
 
 // Operator codes of a coarse level: the fine rules (stencil_code_kernel) without the anchor, except on periodic axes
 // of one or two cells (below). The two spare entries past the end are zero (inactive).
-__global__ void mg_code_kernel(const MgLevel L, const __grid_constant__ StepParams P) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ void code_cell(const MgLevel& L, const StepParams& P, uint32_t q) {
     if (q >= L.n + 2) return;
     if (q >= L.n) {
         L.code[q] = 0;
@@ -1810,9 +1815,23 @@ __global__ void mg_code_kernel(const MgLevel L, const __grid_constant__ StepPara
     L.code[q] = static_cast<uint16_t>(mask | (diag << 8) | kCodeActive);
 }
 
-// Zeroes the two spare entries past the level-0 codes.
-__global__ void mg_code_tail_kernel(uint16_t* code, uint32_t n) {
-    if (threadIdx.x < 2) code[n + threadIdx.x] = 0;
+__global__ void mg_code_kernel(const MgLevel L, const __grid_constant__ StepParams P) {
+    pdl_begin();
+    code_cell(L, P, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// Fluid marks, codes and table entries of the block levels, in one block: with two kernels a level and one for the table the
+// launches of these few hundred cells took longer than the large levels' work (a moving obstacle pays them every frame).
+__global__ void __launch_bounds__(kBlockLevelThreads) mg_block_setup_kernel(const __grid_constant__ MgHierarchy H, const __grid_constant__ StepParams P) {
+    pdl_begin();
+    for (int l = H.grid_levels; l < H.levels; ++l) {
+        for (uint32_t q = threadIdx.x; q < H.L[l].n; q += blockDim.x) coarsen_cell(H.L[l - 1], H.L[l], q);
+        __syncthreads();
+    }
+    for (int l = H.grid_levels; l < H.levels; ++l)
+        for (uint32_t q = threadIdx.x; q < H.L[l].n + 2; q += blockDim.x) code_cell(H.L[l], P, q);
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < H.block_cells; q += blockDim.x) block_table_entry(H, q);
 }
 
 }  // namespace
@@ -1846,13 +1865,12 @@ cudaError_t launch_mg_net_mask(const MgHierarchy& H, uint8_t* solid, cudaStream_
 }
 
 cudaError_t launch_mg_setup(const StepParams& P, const MgHierarchy& H, const uint8_t* occ, cudaStream_t s) {
-    mg_fluid0_kernel<<<(H.L[0].n + 255) / 256, 256, 0, s>>>(H.L[0].n, occ, H.L[0].fluid);
-    mg_code_tail_kernel<<<1, 32, 0, s>>>(H.L[0].code, H.L[0].n);
-    for (int l = 1; l < H.levels; ++l) {
-        mg_coarsen_kernel<<<(H.L[l].n + 255) / 256, 256, 0, s>>>(H.L[l - 1], H.L[l]);
-        mg_code_kernel<<<(H.L[l].n + 2 + 255) / 256, 256, 0, s>>>(H.L[l], P);
+    launch_pdl(mg_fluid0_kernel, (H.L[0].n + 255) / 256, 256, 0, s, H.L[0].n, occ, H.L[0].fluid, H.L[0].code);
+    for (int l = 1; l < H.grid_levels; ++l) {
+        launch_pdl(mg_coarsen_kernel, (H.L[l].n + 255) / 256, 256, 0, s, H.L[l - 1], H.L[l]);
+        launch_pdl(mg_code_kernel, (H.L[l].n + 2 + 255) / 256, 256, 0, s, H.L[l], P);
     }
-    mg_block_table_kernel<<<(H.block_cells + kThreads - 1) / kThreads, kThreads, 0, s>>>(H);
+    launch_pdl(mg_block_setup_kernel, 1, kBlockLevelThreads, 0, s, H, P);
     return cudaGetLastError();
 }
 

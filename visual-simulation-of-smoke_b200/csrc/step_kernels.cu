@@ -564,25 +564,37 @@ __global__ void __launch_bounds__(kThreads) views_kernel(const __grid_constant__
 
 // ------------------------------------------------------------------------------------------ occupancy-derived
 __global__ void occupancy_float_kernel(uint32_t n, const uint8_t* __restrict__ occ, float* __restrict__ out) {
+    pdl_begin();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n) out[q] = static_cast<float>(occ[q]);
 }
 
-__global__ void set_int_kernel(int32_t* p, int32_t v) { *p = v; }
+__global__ void set_int_kernel(int32_t* p, int32_t v) {
+    pdl_begin();
+    *p = v;
+}
 
 // anchor = smallest fluid cell index (:1292-1302); warp minimum first, one atomic per warp.
-__global__ void anchor_kernel(uint32_t n, const uint8_t* __restrict__ occ, int32_t* anchor) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    int32_t v = (q < n && occ[q] == 0) ? static_cast<int32_t>(q) : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0 && v != 0x7fffffff) atomicMin(anchor, v);
+// The first fluid cell into *anchor (set to n before). Warps take runs of 32 cells in ascending order and stop at the first
+// one with a fluid cell or past an anchor already found, so a grid of one block per SM reads little more than the cells up to
+// it (one atomic for each of the grid's warps took 25 us at 96x128x96, now 3).
+__global__ void __launch_bounds__(kThreads) anchor_kernel(uint32_t n, const uint8_t* __restrict__ occ, int32_t* anchor) {
+    pdl_begin();
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kThreads / 32);
+    for (uint64_t first = 32ull * (blockIdx.x * (kThreads / 32) + threadIdx.x / 32); first < n; first += 32ull * warps) {
+        if (static_cast<int64_t>(first) >= *static_cast<volatile int32_t*>(anchor)) return;
+        const uint32_t fluid = __ballot_sync(0xffffffffu, first + lane < n && occ[first + lane] == 0);
+        if (fluid == 0) continue;
+        if (lane == 0) atomicMin(anchor, static_cast<int32_t>(first + __ffs(static_cast<int>(fluid)) - 1u));
+        return;
+    }
 }
 
 // Row code of the Poisson operator (:1343-1412): solid or anchor rows are identity (diag 1, no neighbours);
 // a fluid row's diagonal counts fluid neighbours (anchor included, periodic wrap, repeats counted) plus OUTFLOW
 // domain faces, at least 1; neighbour bits mark distinct fluid non-anchor neighbours other than the cell itself.
 __global__ void __launch_bounds__(kThreads) stencil_code_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor_ptr, uint16_t* __restrict__ codes) {
+    pdl_begin();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= P.n) return;
     const int32_t anchor = *anchor_ptr;
@@ -619,6 +631,7 @@ __global__ void __launch_bounds__(kThreads) stencil_code_kernel(const __grid_con
 
 // The solid cells, in no particular order, each without a source (a warp's cells take one slot range).
 __global__ void __launch_bounds__(kThreads) fill_list_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, FillEntry* __restrict__ list, uint32_t* __restrict__ count) {
+    pdl_begin();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
     const bool solid = q < P.n && occ[q] != 0;
     const uint32_t solids = __ballot_sync(0xffffffffu, solid);
@@ -653,12 +666,15 @@ __device__ __forceinline__ void shell_offset(uint32_t i, int r, int& dx, int& dy
     }
 }
 
+constexpr int kFillBatch = 4;  // neighbours a lane looks at together
+
 // Nearest-fluid source of each solid cell (:1243-1290): first Chebyshev shell (radius 1, 2, ...) holding a fluid cell,
 // smallest squared distance in it, first in (dz, dy, dx) scan order on ties, density periodicity. A cell at depth r has
 // (2 r + 1)^3 neighbours to look at, one load latency after the other if a thread walks them, and the deepest cell decides
 // the time; so a warp takes a cell and its lanes share each shell. The scan order is part of the key that the lanes reduce.
 // A sphere of solid cells in 96 x 128 x 96: 452 us with a thread per cell, 42 with these two kernels.
 __global__ void __launch_bounds__(kThreads) fill_source_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor_ptr, FillEntry* __restrict__ list, const uint32_t* __restrict__ count) {
+    pdl_begin();
     if (*anchor_ptr >= static_cast<int32_t>(P.n)) return;  // no fluid cell exists
     const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kThreads / 32), entries = *count;
     const int max_radius = imax(P.nx, imax(P.ny, P.nz));
@@ -670,26 +686,36 @@ __global__ void __launch_bounds__(kThreads) fill_source_kernel(const __grid_cons
             const uint64_t cells = 24ull * r * r + 2ull;
             int best_d2 = 0x7fffffff;
             uint64_t best_order = ~0ull;
-            for (uint64_t i = lane; i < cells; i += 32u) {
-                int dx, dy, dz;
-                shell_offset(static_cast<uint32_t>(i), r, dx, dy, dz);
-                int c[3] = {x + dx, y + dy, z + dz};
-                const int nn[3] = {P.nx, P.ny, P.nz};
-                bool ok = true;
+            for (uint64_t i0 = lane; i0 < cells; i0 += 32u * kFillBatch) {
+                int d[kFillBatch][3];
+                int32_t cell[kFillBatch];  // -1: outside the domain or solid
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if (P.dper[a]) c[a] = wrapi(c[a], nn[a]);
-                    ok = ok && c[a] >= 0 && c[a] < nn[a];
+                for (int u = 0; u < kFillBatch; ++u) {
+                    const uint64_t i = i0 + 32u * u;
+                    shell_offset(static_cast<uint32_t>(i < cells ? i : 0u), r, d[u][0], d[u][1], d[u][2]);
+                    int c[3] = {x + d[u][0], y + d[u][1], z + d[u][2]};
+                    const int nn[3] = {P.nx, P.ny, P.nz};
+                    bool ok = i < cells;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        if (P.dper[a]) c[a] = wrapi(c[a], nn[a]);
+                        ok = ok && c[a] >= 0 && c[a] < nn[a];
+                    }
+                    cell[u] = ok ? static_cast<int32_t>(cidx(P, c[0], c[1], c[2])) : -1;
                 }
-                if (!ok) continue;
-                const uint32_t nb = cidx(P, c[0], c[1], c[2]);
-                if (occ[nb] != 0) continue;
-                const int d2 = dx * dx + dy * dy + dz * dz;
-                const uint64_t order = (static_cast<uint64_t>(dz + r) << 42) | (static_cast<uint64_t>(dy + r) << 21) | static_cast<uint64_t>(dx + r);
-                if (d2 < best_d2 || (d2 == best_d2 && order < best_order)) {
-                    best_d2 = d2;
-                    best_order = order;
-                    best = static_cast<int32_t>(nb);
+                uint8_t solid[kFillBatch];
+#pragma unroll
+                for (int u = 0; u < kFillBatch; ++u) solid[u] = cell[u] >= 0 ? occ[cell[u]] : 1;
+#pragma unroll
+                for (int u = 0; u < kFillBatch; ++u) {
+                    if (solid[u]) continue;
+                    const int d2 = d[u][0] * d[u][0] + d[u][1] * d[u][1] + d[u][2] * d[u][2];
+                    const uint64_t order = (static_cast<uint64_t>(d[u][2] + r) << 42) | (static_cast<uint64_t>(d[u][1] + r) << 21) | static_cast<uint64_t>(d[u][0] + r);
+                    if (d2 < best_d2 || (d2 == best_d2 && order < best_order)) {
+                        best_d2 = d2;
+                        best_order = order;
+                        best = cell[u];
+                    }
                 }
             }
             for (int o = 16; o > 0; o >>= 1) {
@@ -882,23 +908,23 @@ cudaError_t launch_occupancy_float(const StepParams& P, const uint8_t* occ, floa
 }
 
 cudaError_t launch_anchor(const StepParams& P, const uint8_t* occ, int32_t* anchor, cudaStream_t s) {
-    set_int_kernel<<<1, 1, 0, s>>>(anchor, static_cast<int32_t>(P.n));
-    anchor_kernel<<<blocks_for(P.n), kThreads, 0, s>>>(P.n, occ, anchor);
+    launch_pdl(set_int_kernel, dim3(1), dim3(1), 0, s, anchor, static_cast<int32_t>(P.n));
+    launch_pdl(anchor_kernel, dim3(std::min(148u, blocks_for(P.n))), dim3(kThreads), 0, s, P.n, occ, anchor);
     return cudaGetLastError();
 }
 
 cudaError_t launch_stencil_codes(const StepParams& P, const uint8_t* occ, const int32_t* anchor, uint16_t* codes, cudaStream_t s) {
-    stencil_code_kernel<<<blocks_for(P.n), kThreads, 0, s>>>(P, occ, anchor, codes);
+    launch_pdl(stencil_code_kernel, dim3(blocks_for(P.n)), dim3(kThreads), 0, s, P, occ, anchor, codes);
     return cudaGetLastError();
 }
 
 cudaError_t launch_fill_build(const StepParams& P, const uint8_t* occ, const int32_t* anchor, FillEntry* list, uint32_t* count, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    fill_list_kernel<<<blocks_for(P.n), kThreads, 0, s>>>(P, occ, list, count);
+    launch_pdl(fill_list_kernel, dim3(blocks_for(P.n)), dim3(kThreads), 0, s, P, occ, list, count);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     constexpr unsigned kFillBlocks = 148 * 8;  // one resident wave; the entry count is on the device
-    fill_source_kernel<<<std::min(kFillBlocks, blocks_for(P.n)), kThreads, 0, s>>>(P, occ, anchor, list, count);
+    launch_pdl(fill_source_kernel, dim3(std::min(kFillBlocks, blocks_for(P.n))), dim3(kThreads), 0, s, P, occ, anchor, list, static_cast<const uint32_t*>(count));
     return cudaGetLastError();
 }
 
