@@ -23,6 +23,51 @@ constexpr int kThreads = 256;
 
 inline unsigned blocks_for(uint64_t count, int threads = kThreads) { return static_cast<unsigned>((count + threads - 1) / threads); }
 
+// The step's elementwise kernels call f(q, x, y, z), q linear, for `planes` cells of a column (x, y) per thread: block
+// blockIdx.x takes kThreads consecutive cells of a plane, blockIdx.y a run of planes. planes = 0: one cell, kThreads
+// consecutive ones per block (see column_planes).
+template <class F>
+__device__ __forceinline__ void for_column(const StepParams& P, int planes, F&& f) {
+    const uint32_t slab = static_cast<uint32_t>(P.nx) * P.ny;
+    uint32_t q = blockIdx.x * kThreads + threadIdx.x;
+    int x, y, z, z1;
+    if (planes > 0) {
+        if (q >= slab) return;
+        y = static_cast<int>(P.div_nx.div(q));
+        x = static_cast<int>(q - static_cast<uint32_t>(y) * P.nx);
+        z = blockIdx.y * planes;
+        z1 = imin(z + planes, P.nz);
+        q += static_cast<uint32_t>(z) * slab;
+    } else {
+        if (q >= P.n) return;
+        cell_xyz(P, q, x, y, z);
+        z1 = z + 1;
+    }
+#pragma unroll 1
+    for (; z < z1; ++z, q += slab) f(q, x, y, z);
+}
+// The same over the faces of axis A, with the block's index b along the plane.
+template <int A, class F>
+__device__ __forceinline__ void for_face_column(const StepParams& P, unsigned b, int planes, F&& f) {
+    const uint32_t sx = fsx<A>(P), slab = sx * fsy<A>(P);
+    uint32_t q = b * kThreads + threadIdx.x;
+    int i, j, k, k1;
+    if (planes > 0) {
+        if (q >= slab) return;
+        j = static_cast<int>(P.div_fx[A].div(q));
+        i = static_cast<int>(q - static_cast<uint32_t>(j) * sx);
+        k = blockIdx.y * planes;
+        k1 = imin(k + planes, fsz<A>(P));
+        q += static_cast<uint32_t>(k) * slab;
+    } else {
+        if (q >= (A == 0 ? P.nu : (A == 1 ? P.nv : P.nw))) return;
+        face_ijk<A>(P, q, i, j, k);
+        k1 = k + 1;
+    }
+#pragma unroll 1
+    for (; k < k1; ++k, q += slab) f(q, i, j, k);
+}
+
 // Flow-resolved cell lookup: wraps periodic axes, false when outside a non-periodic domain (:146-151).
 __device__ __forceinline__ bool resolve_flow(const StepParams& P, int& x, int& y, int& z) {
     if (P.fper[0]) x = wrapi(x, P.nx);
@@ -183,9 +228,7 @@ __global__ void __launch_bounds__(kThreads) cell_force_kernel(const __grid_const
 }
 
 template <int A>
-__device__ __forceinline__ void face_force_one(const StepParams& P, uint32_t q, const float* __restrict__ in, const float* __restrict__ f, const uint8_t* __restrict__ occ, const float* __restrict__ solid, float* __restrict__ out, float* __restrict__ pad) {
-    int i, j, k;
-    face_ijk<A>(P, q, i, j, k);
+__device__ __forceinline__ void face_force_one(const StepParams& P, uint32_t q, int i, int j, int k, const float* __restrict__ in, const float* __restrict__ f, const uint8_t* __restrict__ occ, const float* __restrict__ solid, float* __restrict__ out, float* __restrict__ pad) {
     // the settled value, also into the interior of the padded copy that the velocity advection reads
     auto put = [&](float v) {
         out[q] = v;
@@ -235,18 +278,15 @@ __device__ __forceinline__ void face_force_one(const StepParams& P, uint32_t q, 
 
 // Block ranges: [0, bu) -> x faces, [bu, bu+bv) -> y faces, rest -> z faces.
 __global__ void __launch_bounds__(kThreads) face_force_kernel(const __grid_constant__ StepParams P, const float* __restrict__ iu, const float* __restrict__ iv, const float* __restrict__ iw, const float* __restrict__ fx, const float* __restrict__ fy, const float* __restrict__ fz, const uint8_t* __restrict__ occ, const float* __restrict__ su,
-                                                               const float* __restrict__ sv, const float* __restrict__ sw, float* __restrict__ ou, float* __restrict__ ov, float* __restrict__ ow, float* __restrict__ pu, float* __restrict__ pv, float* __restrict__ pw, unsigned bu, unsigned bv) {
+                                                               const float* __restrict__ sv, const float* __restrict__ sw, float* __restrict__ ou, float* __restrict__ ov, float* __restrict__ ow, float* __restrict__ pu, float* __restrict__ pv, float* __restrict__ pw, unsigned bu, unsigned bv, int planes) {
     pdl_begin();
     const unsigned b = blockIdx.x;
     if (b < bu) {
-        const uint32_t q = b * kThreads + threadIdx.x;
-        if (q < P.nu) face_force_one<0>(P, q, iu, fx, occ, su, ou, pu);
+        for_face_column<0>(P, b, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<0>(P, q, i, j, k, iu, fx, occ, su, ou, pu); });
     } else if (b < bu + bv) {
-        const uint32_t q = (b - bu) * kThreads + threadIdx.x;
-        if (q < P.nv) face_force_one<1>(P, q, iv, fy, occ, sv, ov, pv);
+        for_face_column<1>(P, b - bu, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<1>(P, q, i, j, k, iv, fy, occ, sv, ov, pv); });
     } else {
-        const uint32_t q = (b - bu - bv) * kThreads + threadIdx.x;
-        if (q < P.nw) face_force_one<2>(P, q, iw, fz, occ, sw, ow, pw);
+        for_face_column<2>(P, b - bu - bv, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<2>(P, q, i, j, k, iw, fz, occ, sw, ow, pw); });
     }
 }
 
@@ -399,35 +439,31 @@ __global__ void __launch_bounds__(256) pad_ghost_kernel(const __grid_constant__ 
 
 // ------------------------------------------------------------------------------------------ pressure rhs
 // b = -(h^2/dt) div u* + sum of OUTFLOW face pressures; 0 at solid cells and at the anchor (:1304-1328).
-__global__ void __launch_bounds__(kThreads) rhs_kernel(const __grid_constant__ StepParams P, const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor, float* __restrict__ rhs) {
+__global__ void __launch_bounds__(kThreads) rhs_kernel(const __grid_constant__ StepParams P, const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor, float* __restrict__ rhs, int planes) {
     pdl_begin();
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= P.n) return;
-    // every load is issued before the anchor/solid test (the six faces of a cell always exist)
-    const bool zero = static_cast<int32_t>(q) == __ldg(anchor) || occ[q] != 0;
-    int x, y, z;
-    cell_xyz(P, q, x, y, z);
-    const float h = P.h;
-    const float div = (u[fidx<0>(P, x + 1, y, z)] - u[fidx<0>(P, x, y, z)] + v[fidx<1>(P, x, y + 1, z)] - v[fidx<1>(P, x, y, z)] + w[fidx<2>(P, x, y, z + 1)] - w[fidx<2>(P, x, y, z)]) * P.inv_h;
-    if (zero) {
-        rhs[q] = 0.0f;
-        return;
-    }
-    float bsum = 0.0f;
-    if (x == 0 && P.flow[0].type == kFlowOutflow) bsum += P.flow[0].pressure;
-    if (x == P.nx - 1 && P.flow[1].type == kFlowOutflow) bsum += P.flow[1].pressure;
-    if (y == 0 && P.flow[2].type == kFlowOutflow) bsum += P.flow[2].pressure;
-    if (y == P.ny - 1 && P.flow[3].type == kFlowOutflow) bsum += P.flow[3].pressure;
-    if (z == 0 && P.flow[4].type == kFlowOutflow) bsum += P.flow[4].pressure;
-    if (z == P.nz - 1 && P.flow[5].type == kFlowOutflow) bsum += P.flow[5].pressure;
-    rhs[q] = -(h * h / P.dt) * div + bsum;
+    for_column(P, planes, [&](uint32_t q, int x, int y, int z) {
+        // every load is issued before the anchor/solid test (the six faces of a cell always exist)
+        const bool zero = static_cast<int32_t>(q) == __ldg(anchor) || occ[q] != 0;
+        const float h = P.h;
+        const float div = (u[fidx<0>(P, x + 1, y, z)] - u[fidx<0>(P, x, y, z)] + v[fidx<1>(P, x, y + 1, z)] - v[fidx<1>(P, x, y, z)] + w[fidx<2>(P, x, y, z + 1)] - w[fidx<2>(P, x, y, z)]) * P.inv_h;
+        if (zero) {
+            rhs[q] = 0.0f;
+            return;
+        }
+        float bsum = 0.0f;
+        if (x == 0 && P.flow[0].type == kFlowOutflow) bsum += P.flow[0].pressure;
+        if (x == P.nx - 1 && P.flow[1].type == kFlowOutflow) bsum += P.flow[1].pressure;
+        if (y == 0 && P.flow[2].type == kFlowOutflow) bsum += P.flow[2].pressure;
+        if (y == P.ny - 1 && P.flow[3].type == kFlowOutflow) bsum += P.flow[3].pressure;
+        if (z == 0 && P.flow[4].type == kFlowOutflow) bsum += P.flow[4].pressure;
+        if (z == P.nz - 1 && P.flow[5].type == kFlowOutflow) bsum += P.flow[5].pressure;
+        rhs[q] = -(h * h / P.dt) * div + bsum;
+    });
 }
 
 // ------------------------------------------------------------------------------------------ projection
 template <int A>
-__device__ __forceinline__ void project_one(const StepParams& P, uint32_t q, const float* __restrict__ in, const float* __restrict__ p, const double* __restrict__ p64, const uint8_t* __restrict__ occ, const float* __restrict__ solid, float* __restrict__ out, float* __restrict__ pad) {
-    int i, j, k;
-    face_ijk<A>(P, q, i, j, k);
+__device__ __forceinline__ void project_one(const StepParams& P, uint32_t q, int i, int j, int k, const float* __restrict__ in, const float* __restrict__ p, const double* __restrict__ p64, const uint8_t* __restrict__ occ, const float* __restrict__ solid, float* __restrict__ out, float* __restrict__ pad) {
     // the projected value, also into the interior of the padded copy that the scalar advection reads
     auto put = [&](float v) {
         out[q] = v;
@@ -478,18 +514,15 @@ __device__ __forceinline__ void project_one(const StepParams& P, uint32_t q, con
 }
 
 __global__ void __launch_bounds__(kThreads) project_kernel(const __grid_constant__ StepParams P, const float* __restrict__ iu, const float* __restrict__ iv, const float* __restrict__ iw, const float* __restrict__ p, const double* __restrict__ p64, const uint8_t* __restrict__ occ, const float* __restrict__ su, const float* __restrict__ sv, const float* __restrict__ sw, float* __restrict__ ou,
-                                                            float* __restrict__ ov, float* __restrict__ ow, float* __restrict__ pu, float* __restrict__ pv, float* __restrict__ pw, unsigned bu, unsigned bv) {
+                                                            float* __restrict__ ov, float* __restrict__ ow, float* __restrict__ pu, float* __restrict__ pv, float* __restrict__ pw, unsigned bu, unsigned bv, int planes) {
     pdl_begin();
     const unsigned b = blockIdx.x;
     if (b < bu) {
-        const uint32_t q = b * kThreads + threadIdx.x;
-        if (q < P.nu) project_one<0>(P, q, iu, p, p64, occ, su, ou, pu);
+        for_face_column<0>(P, b, planes, [&](uint32_t q, int i, int j, int k) { project_one<0>(P, q, i, j, k, iu, p, p64, occ, su, ou, pu); });
     } else if (b < bu + bv) {
-        const uint32_t q = (b - bu) * kThreads + threadIdx.x;
-        if (q < P.nv) project_one<1>(P, q, iv, p, p64, occ, sv, ov, pv);
+        for_face_column<1>(P, b - bu, planes, [&](uint32_t q, int i, int j, int k) { project_one<1>(P, q, i, j, k, iv, p, p64, occ, sv, ov, pv); });
     } else {
-        const uint32_t q = (b - bu - bv) * kThreads + threadIdx.x;
-        if (q < P.nw) project_one<2>(P, q, iw, p, p64, occ, sw, ow, pw);
+        for_face_column<2>(P, b - bu - bv, planes, [&](uint32_t q, int i, int j, int k) { project_one<2>(P, q, i, j, k, iw, p, p64, occ, sw, ow, pw); });
     }
 }
 
@@ -739,6 +772,9 @@ __global__ void fill_value_kernel(float* __restrict__ dst, float value, uint64_t
 
 }  // namespace
 
+constexpr uint32_t kColumnCells = 600000, kColumnSlab = 16 * kThreads;
+constexpr int kColumnPlanes = 4;
+
 StepParams make_params(const SmokeSimulationConfig& cfg) {
     StepParams P{};
     P.nx = cfg.nx;
@@ -792,6 +828,29 @@ bool set_advect_tile(StepParams& P, int code) {
     return true;
 }
 
+// Cells of a column per thread in the projection, face-force and right-hand-side kernels (for_column). They are bound
+// by instruction issue, a good part of it index arithmetic, which a column pays once: 256x384x256 face force 453 -> 333 us,
+// projection 365 -> 271, right-hand side 142 -> 119; 128^3 34 -> 30, 30 -> 25, 13 -> 10. Two cells
+// give half of that, 8 or 16 leave 97x141x83 too few threads (projection 20, 21, 26 and 41 us with 2, 4, 8 and 16). Below
+// kColumnCells (32^3 would keep 4 blocks busy) and on thin planes, which would fill their blocks badly, a thread takes one
+// cell. Vorticity and cell force got slower as columns (30 -> 40 and 22 -> 27 us at 97x141x83) and stay with one.
+int column_planes(const StepParams& P) { return P.n >= kColumnCells && static_cast<uint32_t>(P.nx) * P.ny >= kColumnSlab ? std::max(kColumnPlanes, (P.nz + 65535) / 65535) : 0; }
+dim3 column_grid(const StepParams& P, int planes) { return planes > 0 ? dim3(blocks_for(static_cast<uint64_t>(P.nx) * P.ny), (P.nz + planes - 1) / planes) : dim3(blocks_for(P.n)); }
+
+// Blocks of the u and v faces and the whole grid of a kernel over all faces.
+struct FaceBlocks {
+    unsigned u, v;
+    dim3 grid;
+};
+FaceBlocks face_blocks(const StepParams& P, int planes) {
+    const uint64_t nx = P.nx, ny = P.ny;
+    FaceBlocks B;
+    B.u = planes > 0 ? blocks_for((nx + 1) * ny) : blocks_for(P.nu);
+    B.v = planes > 0 ? blocks_for(nx * (ny + 1)) : blocks_for(P.nv);
+    B.grid = planes > 0 ? dim3(B.u + B.v + blocks_for(nx * ny), (P.nz + planes) / planes) : dim3(B.u + B.v + blocks_for(P.nw));
+    return B;
+}
+
 cudaError_t launch_vorticity(const StepParams& P, ConstFaces vel, const uint8_t* occ, float* wx, float* wy, float* wz, float* wmag, cudaStream_t s) {
     vorticity_kernel<<<blocks_for(P.n), kThreads, 0, s>>>(P, vel.u, vel.v, vel.w, occ, wx, wy, wz, wmag);
     return cudaGetLastError();
@@ -803,8 +862,9 @@ cudaError_t launch_cell_force(const StepParams& P, const float* wx, const float*
 }
 
 cudaError_t launch_face_force(const StepParams& P, ConstFaces in, const float* fx, const float* fy, const float* fz, const uint8_t* occ, ConstFaces solid, Faces out, cudaStream_t s, Faces pad) {
-    const unsigned bu = blocks_for(P.nu), bv = blocks_for(P.nv), bw = blocks_for(P.nw);
-    launch_pdl(face_force_kernel, dim3(bu + bv + bw), dim3(kThreads), 0, s, P, in.u, in.v, in.w, fx, fy, fz, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, bu, bv);
+    const int planes = column_planes(P);
+    const FaceBlocks B = face_blocks(P, planes);
+    launch_pdl(face_force_kernel, B.grid, dim3(kThreads), 0, s, P, in.u, in.v, in.w, fx, fy, fz, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, B.u, B.v, planes);
     return cudaGetLastError();
 }
 
@@ -873,13 +933,15 @@ cudaError_t launch_advect_velocity(const StepParams& P, ConstFaces in, ConstFace
 }
 
 cudaError_t launch_rhs(const StepParams& P, ConstFaces vel, const uint8_t* occ, const int32_t* anchor, float* rhs, cudaStream_t s) {
-    launch_pdl(rhs_kernel, dim3(blocks_for(P.n)), dim3(kThreads), 0, s, P, vel.u, vel.v, vel.w, occ, anchor, rhs);
+    const int planes = column_planes(P);
+    launch_pdl(rhs_kernel, column_grid(P, planes), dim3(kThreads), 0, s, P, vel.u, vel.v, vel.w, occ, anchor, rhs, planes);
     return cudaGetLastError();
 }
 
 cudaError_t launch_project(const StepParams& P, ConstFaces in, const float* pressure, const double* pressure64, const uint8_t* occ, ConstFaces solid, Faces out, cudaStream_t s, Faces pad) {
-    const unsigned bu = blocks_for(P.nu), bv = blocks_for(P.nv), bw = blocks_for(P.nw);
-    launch_pdl(project_kernel, dim3(bu + bv + bw), dim3(kThreads), 0, s, P, in.u, in.v, in.w, pressure, pressure64, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, bu, bv);
+    const int planes = column_planes(P);
+    const FaceBlocks B = face_blocks(P, planes);
+    launch_pdl(project_kernel, B.grid, dim3(kThreads), 0, s, P, in.u, in.v, in.w, pressure, pressure64, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, B.u, B.v, planes);
     return cudaGetLastError();
 }
 
