@@ -30,10 +30,23 @@ SHAPES = [
 ]
 
 
+# 2 to 16 blocks run as one cluster, whatever the count; 17 do not
+CLUSTERS = [(32, 8, 8 * blocks) for blocks in (2, 3, 5, 6, 7, 8, 9, 11, 13, 14, 15, 16, 17)]
+
+
 @pytest.mark.parametrize("boundary", ["closed", "plume", "zout"])
 @pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
 @pytest.mark.parametrize("reduction", [abi.REDUCTION_FP32, abi.REDUCTION_FP64], ids=["fp32", "fp64"])
 def test_fixed_cg_on_chip_matches_oracle(smoke_lib, cuda_stream, shape, boundary, reduction):
+    check_against_oracle(smoke_lib, cuda_stream, shape, boundary, reduction)
+
+
+@pytest.mark.parametrize("shape", CLUSTERS, ids=["x".join(map(str, s)) for s in CLUSTERS])
+def test_fixed_cg_in_one_cluster_matches_oracle(smoke_lib, cuda_stream, shape):
+    check_against_oracle(smoke_lib, cuda_stream, shape, "plume", abi.REDUCTION_FP32)
+
+
+def check_against_oracle(smoke_lib, cuda_stream, shape, boundary, reduction):
     cfg = scenes.make_config(*shape, boundary=boundary, mode=abi.LINEAR, pressure_iterations=10)
     inp = scenes.random_inputs(cfg, seed=sum(shape), solids=shape[0] != 32)
     sim = smoke_b200.Simulation(smoke_lib, cfg, cuda_stream)

@@ -522,29 +522,55 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     }
 }
 
+// Grids of at most 16 blocks run as one thread-block cluster: its blocks are resident together by definition, and on
+// neighbouring SMs, where a word is on its way for less time (32^3, 16 blocks: a step 468 -> 374 us; the cluster lands on either die, and a solve
+// takes 283 or 410 us by where the words are homed).
+constexpr int kClusterBlocks = 16;
+
 template <typename T, int M>
 cudaError_t launch_one(const ResidentArgs& A, cudaStream_t s) {
     static std::mutex lock;
-    static std::map<int, cudaError_t> configured;  // per device
+    static std::map<int, cudaError_t> configured;            // per device
+    static std::map<std::pair<int, int>, bool> one_cluster;  // per device and block count
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    {
-        std::lock_guard<std::mutex> guard(lock);
-        auto it = configured.find(dev);
-        if (it == configured.end()) it = configured.emplace(dev, cudaFuncSetAttribute(pcg_resident_kernel<T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(resident_smem(M)))).first;
-        if (it->second != cudaSuccess) return it->second;
-    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(A.plan.blocks);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = resident_smem(A.plan.planes);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    bool cluster = false;
+    {
+        std::lock_guard<std::mutex> guard(lock);
+        auto it = configured.find(dev);
+        if (it == configured.end()) {
+            e = cudaFuncSetAttribute(pcg_resident_kernel<T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(resident_smem(M)));
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(pcg_resident_kernel<T, M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            it = configured.emplace(dev, e).first;
+        }
+        if (it->second != cudaSuccess) return it->second;
+        if (A.plan.blocks > 1 && A.plan.blocks <= kClusterBlocks) {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim = {static_cast<unsigned>(A.plan.blocks), 1u, 1u};
+            auto c = one_cluster.find({dev, A.plan.blocks});
+            if (c == one_cluster.end()) {
+                int clusters = 0;
+                const bool ok = cudaOccupancyMaxActiveClusters(&clusters, pcg_resident_kernel<T, M>, &cfg) == cudaSuccess && clusters > 0;
+                if (!ok) cudaGetLastError();  // a block count the device does not take as a cluster
+                c = one_cluster.emplace(std::make_pair(dev, A.plan.blocks), ok).first;
+            }
+            cluster = c->second;
+        }
+    }
+    if (!cluster) {
+        attr[0] = cudaLaunchAttribute{};
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    }
     return cudaLaunchKernelEx(&cfg, pcg_resident_kernel<T, M>, A);
 }
 
