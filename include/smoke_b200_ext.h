@@ -134,10 +134,10 @@ typedef struct SmokeB200LaunchTune {
                               1: 32x8x1, 2: 32x4x2, 3: 16x4x4, 4: 8x8x4 faces or cells */
     uint32_t mg_wave;      /* multigrid level kernels, grid depth: 0, 1 (default), 2, 3: 1/2, 1, 2, 4 waves of
                               resident blocks; 4: one block per 32x4x2 tile */
-    uint32_t pcg_grid;     /* persistent CG kernel (FIXED_CG, JACOBI_PCG): 0 all resident blocks (default), 1 half,
-                              2 a quarter */
-    uint32_t pcg_regs;     /* persistent CG kernel: 0 compiled without a register cap (default, 2 blocks per SM),
-                              1 capped at 64 registers (4 blocks per SM, more loads in flight, a few spills) */
+    uint32_t pcg_grid;     /* streaming CG kernel (JACOBI_PCG, and FIXED_CG on grids that do not fit on the chip): 0 all
+                              resident blocks (default), 1 half, 2 a quarter */
+    uint32_t pcg_regs;     /* streaming CG kernel: 0 compiled without a register cap (default, 1 block per SM), 1 capped at
+                              64 registers (4 blocks per SM, more loads in flight, a few spills) */
 } SmokeB200LaunchTune;
 
 /* One timed candidate of smoke_b200_autotune_cuda. */

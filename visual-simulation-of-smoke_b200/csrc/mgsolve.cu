@@ -1534,7 +1534,7 @@ dim3 wave(K kernel, const MgLevel& L, int depth) {
 }
 
 // Rows of a thread of a level-0 z-march kernel: 4, or 2 where 4 would leave a warp of the chip's one wave without a plane
-// pair of its own.
+// pair of its own (an iteration with 4 and with 2: 67.3 and 63.5 us at 64^3, 118 and 120 at 128^3, 765 and 867 at 256x384x256).
 constexpr uint32_t kMarchWideCells = 80u * 80u * 80u;
 inline int march_rows(const MgLevel& L) { return L.n >= kMarchWideCells ? 4 : 2; }
 

@@ -85,7 +85,7 @@ struct X64Data {
 template <typename T>
 __device__ __forceinline__ bool finite_all(T a, T b, T c) { return isfinite(a) && isfinite(b) && isfinite(c); }
 
-// MINB: blocks per SM the register allocation must allow (1: unconstrained, about 125 registers and 2 blocks per SM;
+// MINB: blocks per SM the register allocation must allow (1: unconstrained, 145-162 registers and one block per SM;
 // 4: at most 64 registers, a few spills, twice the loads in flight; the autotuner picks per grid).
 template <bool JACOBI, typename T, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) pcg_kernel(const __grid_constant__ StepParams P, const PcgSettings S, const Columns C, const uint16_t* __restrict__ codes, const float* __restrict__ b, float* x, PcgWork W, PcgControl* ctl) {

@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kEpiThreads) wgrad_kernel(const __grid_constan
 
 // grad[w(tap, ci, co)] (+)= sum over blocks of partial[b][tap * cs + ci][co]; grad[bias co] likewise from row
 // 27 * cs. The sum runs over the blocks in order, eight loads in flight at a time (one by one, each waited for L2: 11 us a
-// layer on a 32^3 sample, now 4).
+// layer on a 32^3 sample).
 __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int blocks, int m_pad, int gn, int cs, int cin, int cout, int accumulate, float* __restrict__ grad) {
     pdl_trigger();
     pdl_wait();
