@@ -7,6 +7,9 @@ Tolerance: FP32 vectors, FP64 dot products and 10 iterations. An iteration round
 the operator about seven times; carried through 10 iterations of growing search directions (at most a factor of ten) that is
 10 * 11 * 6e-8 * 10 < 1e-4 of the largest pressure.
 """
+import ctypes as C
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -66,3 +69,37 @@ def check_against_oracle(smoke_lib, cuda_stream, shape, boundary, reduction):
     assert status.iterations == 10 and status.status == abi.SOLVE_ITERATION_CAP
     assert np.array_equal(p, again)
     assert scenes.rel_err(p, x) < 1e-4
+
+
+# the iterations whose halo waits run out: the first and one in the middle
+@pytest.mark.parametrize("exchange", [1, 5])
+@pytest.mark.parametrize("shape,block", [((32, 8, 40), 2), ((48, 40, 32), 1), ((96, 96, 96), 70)], ids=["cluster", "grid", "planes24"])
+def test_halo_wait_that_runs_out_aborts_the_solve(smoke_lib, cuda_stream, shape, block, exchange):
+    """A block whose neighbours never get its faces of one exchange: their bounded waits run out, every block leaves, the
+    status says so, and the next solve on the context gives the bits of the one before."""
+    cfg = scenes.make_config(*shape, boundary="plume", mode=abi.LINEAR, pressure_iterations=10)
+    inp = scenes.random_inputs(cfg, seed=sum(shape), solids=False)
+    sim = smoke_b200.Simulation(smoke_lib, cfg, cuda_stream)
+    keep = scenes.load_gpu(sim, inp)
+    sim.set_solver(abi.SOLVER_FIXED_CG, abi.REDUCTION_FP32)
+    with torch.cuda.stream(cuda_stream):
+        sim.step_stages(abi.STAGE_PRESSURE)
+    p = sim.snapshot([abi.VIEW_FLOW_PRESSURE])["pressure"]
+    st = abi.SolverStatus()
+    hook = smoke_lib.lib.smoke_b200_test_exchange_timeout_cuda
+    t0 = time.perf_counter()
+    assert hook(sim.handle, block, exchange, 100, C.byref(st)) == abi.RESULT_OK
+    waited = time.perf_counter() - t0
+    assert st.status == abi.SOLVE_BARRIER_TIMEOUT, st.status
+    assert 0.05 < waited < 5.0, waited
+    with torch.cuda.stream(cuda_stream):
+        sim.solve_pressure()
+    again = sim.snapshot([abi.VIEW_FLOW_PRESSURE])["pressure"]
+    status = sim.solver_status()
+    assert status.iterations == 10 and status.status == abi.SOLVE_ITERATION_CAP
+    assert np.array_equal(p, again)
+    assert hook(sim.handle, block, 0, 100, C.byref(st)) == abi.RESULT_BACKEND_FAILURE
+    sim.set_solver(abi.SOLVER_JACOBI_PCG, abi.REDUCTION_FP64, max_iterations=100, tolerance=1e-5)
+    assert hook(sim.handle, block, 1, 100, C.byref(st)) == abi.RESULT_BACKEND_FAILURE  # no exchange of faces there
+    sim.close()
+    del keep

@@ -499,6 +499,21 @@ cudaError_t copy_or_zero(float* dst, const float* src, size_t count, cudaStream_
     return cudaMemcpyAsync(dst, src, count * sizeof(float), cudaMemcpyDeviceToDevice, s);
 }
 
+// The context's persistent solve with a block withheld (exchange > 0: only its faces of that exchange), and its status.
+SmokeSimulationResult solve_withheld(SmokeSimulationContext_t& c, uint32_t block, uint32_t exchange, uint32_t timeout_ms, SmokeB200SolverStatus* out) {
+    PcgSettings S = c.pcg_settings();
+    S.withhold_block = static_cast<int32_t>(block) + 1;
+    S.withhold_exchange = static_cast<int32_t>(exchange);
+    S.barrier_timeout_ms = timeout_ms;
+    check(launch_pcg(c.P, S, c.pcg_shape, c.codes, c.rhs, c.pressure, c.pcg, c.control, c.stream), "pressure solve with a withheld block");
+    c.stepped = true;
+    PcgStatusDevice st{};
+    check(cudaMemcpyAsync(&st, &c.control->status, sizeof(st), cudaMemcpyDeviceToHost, c.stream), "status read-back");
+    check(cudaStreamSynchronize(c.stream), "status read-back");
+    std::memcpy(out, &st, sizeof(st));
+    return SMOKE_SIMULATION_RESULT_OK;
+}
+
 // ---------------------------------------------------------------------------------------------- autotuner
 // Tuned shapes, per process: (device, nx, ny, nz, cubic, solver mode, reduction, refinement, max iterations,
 // tolerance bits).
@@ -779,18 +794,13 @@ SmokeSimulationResult smoke_b200_step_stages_cuda(SmokeSimulationContext c, uint
 
 SmokeSimulationResult smoke_b200_test_barrier_timeout_cuda(SmokeSimulationContext c, uint32_t block, uint32_t timeout_ms, SmokeB200SolverStatus* out_status) {
     if (c == nullptr || out_status == nullptr || block == 0 || timeout_ms == 0 || timeout_ms > 10000 || c->uses_mg()) return SMOKE_SIMULATION_RESULT_BACKEND_FAILURE;
-    return guarded([&] {
-        PcgSettings S = c->pcg_settings();
-        S.withhold_block = static_cast<int32_t>(block) + 1;
-        S.barrier_timeout_ms = timeout_ms;
-        check(launch_pcg(c->P, S, c->pcg_shape, c->codes, c->rhs, c->pressure, c->pcg, c->control, c->stream), "pressure solve with a withheld block");
-        c->stepped = true;
-        PcgStatusDevice st{};
-        check(cudaMemcpyAsync(&st, &c->control->status, sizeof(st), cudaMemcpyDeviceToHost, c->stream), "status read-back");
-        check(cudaStreamSynchronize(c->stream), "status read-back");
-        std::memcpy(out_status, &st, sizeof(st));
-        return SMOKE_SIMULATION_RESULT_OK;
-    });
+    return guarded([&] { return solve_withheld(*c, block, 0, timeout_ms, out_status); });
+}
+
+SmokeSimulationResult smoke_b200_test_exchange_timeout_cuda(SmokeSimulationContext c, uint32_t block, uint32_t exchange, uint32_t timeout_ms, SmokeB200SolverStatus* out_status) {
+    if (c == nullptr || out_status == nullptr || exchange == 0 || exchange > 0x7fffffffu || timeout_ms == 0 || timeout_ms > 10000) return SMOKE_SIMULATION_RESULT_BACKEND_FAILURE;
+    if (!pcg_runs_resident(c->pcg_settings(), c->pcg_shape, c->pcg)) return SMOKE_SIMULATION_RESULT_BACKEND_FAILURE;
+    return guarded([&] { return solve_withheld(*c, block, exchange, timeout_ms, out_status); });
 }
 
 SmokeSimulationResult smoke_b200_solve_pressure_cuda(SmokeSimulationContext c) {

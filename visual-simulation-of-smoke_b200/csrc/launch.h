@@ -104,7 +104,7 @@ struct PcgSettings {
     int32_t warm_start;      // start from x instead of 0
     int32_t withhold_block;  // test only: > 0 makes block withhold_block - 1 leave before its first grid barrier
     uint32_t barrier_timeout_ms;  // bound of every grid-barrier wait (0: the default, 2000 ms)
-    uint32_t pad;
+    int32_t withhold_exchange;  // test only, resident kernel: > 0 lets that block run and withhold its faces of this exchange
 };
 
 struct PcgStatusDevice {
@@ -273,6 +273,8 @@ cudaError_t run_mg_solve_eager(const MgSolveArgs& args, bool fp64, PcgStatusDevi
 
 // Picks the persistent grid (all blocks co-resident) for the current device.
 cudaError_t pcg_launch_shape(const StepParams& P, PcgLaunchShape* out);
+// Whether launch_pcg runs the solve on the chip.
+bool pcg_runs_resident(const PcgSettings& S, const PcgLaunchShape& shape, const PcgWork& work);
 // The fixed-count solve with its state on the chip (pcg_resident.cu).
 cudaError_t launch_pcg_resident(const StepParams& P, const PcgSettings& S, const PcgResidentPlan& plan, const uint16_t* codes, const float* b, float* x, const PcgWork& work, PcgControl* ctl, cudaStream_t s);
 // Enqueues: reset of the control header, then the cooperative solver launch.

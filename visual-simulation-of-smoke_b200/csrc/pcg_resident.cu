@@ -56,7 +56,9 @@ __device__ __forceinline__ void get_words(const unsigned long long* p, unsigned 
 }
 __device__ __forceinline__ uint32_t tag_of(unsigned long long v) { return static_cast<uint32_t>(v >> 32); }
 
-// A wait's bound, and where giving up is recorded (the grid's abort word, the block's flag).
+// A wait's bound, and where giving up is recorded: the grid's abort word and the block's flag for waits of this kind. Halo
+// waits and sum waits have a flag each: it is read behind the barrier that ends the waits, and another barrier comes before the
+// next waits that may set it, so every warp of the block reads the same value.
 struct Wait {
     PcgControl* ctl;
     int* flag;
@@ -92,6 +94,7 @@ struct ResidentArgs {
     PcgControl* ctl;
     int iterations;
     int withhold_block;
+    int withhold_exchange;
     uint32_t barrier_timeout_ms;
 };
 
@@ -143,9 +146,10 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     extern __shared__ __align__(16) float area[];
     __shared__ T red[kSums][kWarps];
     __shared__ double all[kPcgSumCopies][kSums];
-    __shared__ int flag;
+    __shared__ int flag[2];  // a halo wait, a sum wait of this block gave up
     // test hook: this block never publishes, so the others' bounded waits run out and abort the solve
-    if (A.withhold_block > 0 && static_cast<int>(blockIdx.x) == A.withhold_block - 1) return;
+    const bool withheld = A.withhold_block > 0 && static_cast<int>(blockIdx.x) == A.withhold_block - 1;
+    if (withheld && A.withhold_exchange == 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;  // a warp is a row of the column
     const uint32_t G = gridDim.x, total = A.plan.total;
     const uint32_t ua = static_cast<uint32_t>((static_cast<uint64_t>(blockIdx.x) * total) / G);
@@ -159,7 +163,8 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     float* const ps = rs + kSlab * (m_max + 4);          // p: [planes][256]
     float* const hs = ps + kThreads * m_max;             // s of the side halo: [planes][80]
     uint16_t* const cs = reinterpret_cast<uint16_t*>(hs + kSideWords * m_max);  // codes: [planes][256]
-    const Wait wait{A.ctl, &flag, A.barrier_timeout_ms ? static_cast<unsigned long long>(A.barrier_timeout_ms) * 1000000ull : gsync::kBarrierTimeoutNs};
+    const unsigned long long timeout_ns = A.barrier_timeout_ms ? static_cast<unsigned long long>(A.barrier_timeout_ms) * 1000000ull : gsync::kBarrierTimeoutNs;
+    const Wait halo_wait{A.ctl, &flag[0], timeout_ns}, sum_wait{A.ctl, &flag[1], timeout_ns};
     uint32_t phase = A.ctl->epoch;  // tag of the last exchange
     // geometry of the block's two columns
     struct Column {
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     };
 
     // ------------------------------------------------------------ r = b with its halo, s = p = x = 0, codes
-    if (tid == 0) flag = 0;
+    if (tid < 2) flag[tid] = 0;
     for (int i = tid; i < kSlab * (m_max + 4); i += kThreads) rs[i] = 0.0f;
     __syncthreads();
     float w[M], s[M], sz[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
@@ -290,6 +295,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     T bb = 0, rr = 0, gamma = 0, alpha = 0, beta = 0;
     for (bool first = true;; first = false) {
         const float fa = static_cast<float>(alpha), fb = static_cast<float>(beta);
+        bool halo_failed = false;
         if (!first) {
             // the halo's w were published before the sums that set alpha and beta: the z faces' and the first group of the side
             // faces' are in flight while the own cells advance
@@ -333,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                     const int zs = halo_slot(k, top);
                     if (zs < 0) continue;
                     if (M > 9) zv[k][top] = get_word(z_words(zs));
-                    if (tag_of(zv[k][top]) != phase) zv[k][top] = poll(z_words(zs), phase, wait);
+                    if (tag_of(zv[k][top]) != phase) zv[k][top] = poll(z_words(zs), phase, halo_wait);
                     advance(__uint_as_float(static_cast<uint32_t>(zv[k][top])), fa, fb, sz[k][top], rs[z_plane(k, top) * kSlab + slot]);
                 }
             for (int j0 = j1; j0 < 3 * m; j0 += kItems * kWarps) {
@@ -344,15 +350,18 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                     int word, rslot, hslot;
                     const int col = side_item(j, word, rslot, hslot);
                     if (col < 0) continue;
-                    if (tag_of(v[n]) != phase) v[n] = poll(side_words(col, plane_z(j / 3)) + word, phase, wait);
+                    if (tag_of(v[n]) != phase) v[n] = poll(side_words(col, plane_z(j / 3)) + word, phase, halo_wait);
                     advance(__uint_as_float(static_cast<uint32_t>(v[n])), fa, fb, hs[hslot], rs[rslot]);
                 }
             }
             __syncthreads();
+            halo_failed = *static_cast<volatile int*>(&flag[0]) != 0;
         }
         // w = A r of the own cells, the faces' w published under a new tag; this thread's (r, r) and (w, r) in plane order
         T loc[kSums] = {0, 0};
         ++phase;
+        // test hook: the faces of one exchange (1: the start's) carry a tag that no reader waits for
+        const uint32_t face_tag = withheld && A.withhold_exchange == (first ? 1 : it + 2) ? phase - 1u : phase;
         {
             unsigned long long* const out = side_words(col0, za);  // units are consecutive: plane i's words 80 i further
             const float* r = ra;
@@ -375,8 +384,8 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                     w[i] = v;
                     loc[0] += static_cast<T>(r0) * static_cast<T>(r0);
                     loc[1] += static_cast<T>(v) * static_cast<T>(r0);
-                    if (yw >= 0) put_word(out + i * kSideWords + yw, __float_as_uint(v), phase);
-                    if (xw >= 0) put_word(out + i * kSideWords + xw, __float_as_uint(v), phase);
+                    if (yw >= 0) put_word(out + i * kSideWords + yw, __float_as_uint(v), face_tag);
+                    if (xw >= 0) put_word(out + i * kSideWords + xw, __float_as_uint(v), face_tag);
                 }
                 rm1 = r0;
                 r0 = r1;
@@ -390,15 +399,15 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
             for (int k = 0; k < 2; ++k) {
                 if (!owns(k)) continue;
                 const int lo = k == 0 ? 0 : m0, hi = k == 0 ? m0 - 1 : m - 1;
-                if (lo == 0 && za > 0) put_word(z_words(2 * blockIdx.x), value(lo), phase);
-                if (hi == m - 1 && plane_z(hi) < A.nz - 1) put_word(z_words(2 * blockIdx.x + 1), value(hi), phase);
-                if (A.per[2] && plane_z(lo) == 0) put_word(z_words(col_slot(col0 + k, 0)), value(lo), phase);
-                if (A.per[2] && plane_z(hi) == A.nz - 1) put_word(z_words(col_slot(col0 + k, 1)), value(hi), phase);
+                if (lo == 0 && za > 0) put_word(z_words(2 * blockIdx.x), value(lo), face_tag);
+                if (hi == m - 1 && plane_z(hi) < A.nz - 1) put_word(z_words(2 * blockIdx.x + 1), value(hi), face_tag);
+                if (A.per[2] && plane_z(lo) == 0) put_word(z_words(col_slot(col0 + k, 0)), value(lo), face_tag);
+                if (A.per[2] && plane_z(hi) == A.nz - 1) put_word(z_words(col_slot(col0 + k, 1)), value(hi), face_tag);
                 if (!thin) continue;
                 const Column& c = k == 0 ? c0 : c1;
                 for (int i = lo; i <= hi; ++i) {
-                    if (c.ey == 1 && c.north >= 0) put_word(out + i * kSideWords + CX + lane, value(i), phase);
-                    if (c.ex == 1 && c.east >= 0) put_word(out + i * kSideWords + 2 * CX + CY + warp, value(i), phase);
+                    if (c.ey == 1 && c.north >= 0) put_word(out + i * kSideWords + CX + lane, value(i), face_tag);
+                    if (c.ex == 1 && c.east >= 0) put_word(out + i * kSideWords + 2 * CX + CY + warp, value(i), face_tag);
                 }
             }
         }
@@ -459,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                     for (int k = 0; k < kSums; ++k) get_words(p + 2 * k, v[2 * k], v[2 * k + 1]);
 #pragma unroll
                     for (int k = 0; k < kSumWords; ++k) ok = ok && tag_of(v[k]) == phase;
-                    if (ok || ((spins & 15u) == 0u && give_up(spins, t0, wait))) break;
+                    if (ok || ((spins & 15u) == 0u && give_up(spins, t0, sum_wait))) break;
                 }
 #pragma unroll
                 for (int k = 0; k < kSums; ++k) acc[k] += __hiloint2double(static_cast<int>(v[2 * k + 1]), static_cast<int>(v[2 * k]));
@@ -476,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
         for (int c = 0; c < kPcgSumCopies; ++c)
 #pragma unroll
             for (int k = 0; k < kSums; ++k) sums[k] += static_cast<T>(all[c][k]);
-        if (*reinterpret_cast<volatile int*>(&flag) != 0) {
+        if (halo_failed || *static_cast<volatile int*>(&flag[1]) != 0) {
             status = SMOKE_B200_SOLVE_BARRIER_TIMEOUT;
             break;
         }
@@ -617,6 +626,7 @@ cudaError_t launch_pcg_resident(const StepParams& P, const PcgSettings& S, const
     A.ctl = ctl;
     A.iterations = S.max_iterations;
     A.withhold_block = S.withhold_block;
+    A.withhold_exchange = S.withhold_exchange;
     A.barrier_timeout_ms = S.barrier_timeout_ms;
     const cudaError_t e = cudaMemsetAsync(ctl, 0, kPcgControlResetBytes, s);
     if (e != cudaSuccess) return e;
