@@ -71,8 +71,8 @@ def check_against_oracle(smoke_lib, cuda_stream, shape, boundary, reduction):
     assert scenes.rel_err(p, x) < 1e-4
 
 
-# the iterations whose halo waits run out: the first and one in the middle
-@pytest.mark.parametrize("exchange", [1, 5])
+# the iterations whose halo waits run out: the first, one in the middle and the last, whose sums alone tell the others
+@pytest.mark.parametrize("exchange", [1, 5, 10])
 @pytest.mark.parametrize("shape,block", [((32, 8, 40), 2), ((48, 40, 32), 1), ((96, 96, 96), 70)], ids=["cluster", "grid", "planes24"])
 def test_halo_wait_that_runs_out_aborts_the_solve(smoke_lib, cuda_stream, shape, block, exchange):
     """A block whose neighbours never get its faces of one exchange: their bounded waits run out, every block leaves, the

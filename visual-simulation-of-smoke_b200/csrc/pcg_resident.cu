@@ -295,7 +295,6 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     T bb = 0, rr = 0, gamma = 0, alpha = 0, beta = 0;
     for (bool first = true;; first = false) {
         const float fa = static_cast<float>(alpha), fb = static_cast<float>(beta);
-        bool halo_failed = false;
         if (!first) {
             // the halo's w were published before the sums that set alpha and beta: the z faces' and the first group of the side
             // faces' are in flight while the own cells advance
@@ -355,7 +354,12 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                 }
             }
             __syncthreads();
-            halo_failed = *static_cast<volatile int*>(&flag[0]) != 0;
+            // r's halo is incomplete: leave without publishing, so that no block gets sums formed from it, in the last iteration
+            // either, after which nothing but those sums is waited for
+            if (*static_cast<volatile int*>(&flag[0]) != 0) {
+                status = SMOKE_B200_SOLVE_BARRIER_TIMEOUT;
+                break;
+            }
         }
         // w = A r of the own cells, the faces' w published under a new tag; this thread's (r, r) and (w, r) in plane order
         T loc[kSums] = {0, 0};
@@ -485,7 +489,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
         for (int c = 0; c < kPcgSumCopies; ++c)
 #pragma unroll
             for (int k = 0; k < kSums; ++k) sums[k] += static_cast<T>(all[c][k]);
-        if (halo_failed || *static_cast<volatile int*>(&flag[1]) != 0) {
+        if (*static_cast<volatile int*>(&flag[1]) != 0) {
             status = SMOKE_B200_SOLVE_BARRIER_TIMEOUT;
             break;
         }
