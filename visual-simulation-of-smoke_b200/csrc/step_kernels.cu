@@ -23,49 +23,48 @@ constexpr int kThreads = 256;
 
 inline unsigned blocks_for(uint64_t count, int threads = kThreads) { return static_cast<unsigned>((count + threads - 1) / threads); }
 
-// The step's elementwise kernels call f(q, x, y, z), q linear, for `planes` cells of a column (x, y) per thread: block
-// blockIdx.x takes kThreads consecutive cells of a plane, blockIdx.y a run of planes. planes = 0: one cell, kThreads
-// consecutive ones per block (see column_planes).
-template <class F>
+// The step's elementwise kernels call f(q, x, y, z), q linear, for one cell per thread, kThreads consecutive ones per block, or
+// (COLUMN) for `planes` cells of a column (x, y): block blockIdx.x takes kThreads consecutive cells of a plane, blockIdx.y a run
+// of planes (see column_planes). The form is the kernel's template argument: one kernel that chose between them by `planes`
+// carried the column's loop into the one-cell form (84^3: face force 14.6 -> 15.4 us, projection 9.6 -> 11.2).
+template <bool COLUMN, class F>
 __device__ __forceinline__ void for_column(const StepParams& P, int planes, F&& f) {
-    const uint32_t slab = static_cast<uint32_t>(P.nx) * P.ny;
     uint32_t q = blockIdx.x * kThreads + threadIdx.x;
-    int x, y, z, z1;
-    if (planes > 0) {
+    if constexpr (COLUMN) {
+        const uint32_t slab = static_cast<uint32_t>(P.nx) * P.ny;
         if (q >= slab) return;
-        y = static_cast<int>(P.div_nx.div(q));
-        x = static_cast<int>(q - static_cast<uint32_t>(y) * P.nx);
-        z = blockIdx.y * planes;
-        z1 = imin(z + planes, P.nz);
+        const int y = static_cast<int>(P.div_nx.div(q)), x = static_cast<int>(q - static_cast<uint32_t>(y) * P.nx);
+        int z = blockIdx.y * planes;
+        const int z1 = imin(z + planes, P.nz);
         q += static_cast<uint32_t>(z) * slab;
+#pragma unroll 1
+        for (; z < z1; ++z, q += slab) f(q, x, y, z);
     } else {
         if (q >= P.n) return;
+        int x, y, z;
         cell_xyz(P, q, x, y, z);
-        z1 = z + 1;
+        f(q, x, y, z);
     }
-#pragma unroll 1
-    for (; z < z1; ++z, q += slab) f(q, x, y, z);
 }
 // The same over the faces of axis A, with the block's index b along the plane.
-template <int A, class F>
+template <int A, bool COLUMN, class F>
 __device__ __forceinline__ void for_face_column(const StepParams& P, unsigned b, int planes, F&& f) {
-    const uint32_t sx = fsx<A>(P), slab = sx * fsy<A>(P);
     uint32_t q = b * kThreads + threadIdx.x;
-    int i, j, k, k1;
-    if (planes > 0) {
+    if constexpr (COLUMN) {
+        const uint32_t sx = fsx<A>(P), slab = sx * fsy<A>(P);
         if (q >= slab) return;
-        j = static_cast<int>(P.div_fx[A].div(q));
-        i = static_cast<int>(q - static_cast<uint32_t>(j) * sx);
-        k = blockIdx.y * planes;
-        k1 = imin(k + planes, fsz<A>(P));
+        const int j = static_cast<int>(P.div_fx[A].div(q)), i = static_cast<int>(q - static_cast<uint32_t>(j) * sx);
+        int k = blockIdx.y * planes;
+        const int k1 = imin(k + planes, fsz<A>(P));
         q += static_cast<uint32_t>(k) * slab;
+#pragma unroll 1
+        for (; k < k1; ++k, q += slab) f(q, i, j, k);
     } else {
         if (q >= (A == 0 ? P.nu : (A == 1 ? P.nv : P.nw))) return;
+        int i, j, k;
         face_ijk<A>(P, q, i, j, k);
-        k1 = k + 1;
+        f(q, i, j, k);
     }
-#pragma unroll 1
-    for (; k < k1; ++k, q += slab) f(q, i, j, k);
 }
 
 // Flow-resolved cell lookup: wraps periodic axes, false when outside a non-periodic domain (:146-151).
@@ -277,16 +276,17 @@ __device__ __forceinline__ void face_force_one(const StepParams& P, uint32_t q, 
 }
 
 // Block ranges: [0, bu) -> x faces, [bu, bu+bv) -> y faces, rest -> z faces.
+template <bool COLUMN>
 __global__ void __launch_bounds__(kThreads) face_force_kernel(const __grid_constant__ StepParams P, const float* __restrict__ iu, const float* __restrict__ iv, const float* __restrict__ iw, const float* __restrict__ fx, const float* __restrict__ fy, const float* __restrict__ fz, const uint8_t* __restrict__ occ, const float* __restrict__ su,
                                                                const float* __restrict__ sv, const float* __restrict__ sw, float* __restrict__ ou, float* __restrict__ ov, float* __restrict__ ow, float* __restrict__ pu, float* __restrict__ pv, float* __restrict__ pw, unsigned bu, unsigned bv, int planes) {
     pdl_begin();
     const unsigned b = blockIdx.x;
     if (b < bu) {
-        for_face_column<0>(P, b, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<0>(P, q, i, j, k, iu, fx, occ, su, ou, pu); });
+        for_face_column<0, COLUMN>(P, b, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<0>(P, q, i, j, k, iu, fx, occ, su, ou, pu); });
     } else if (b < bu + bv) {
-        for_face_column<1>(P, b - bu, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<1>(P, q, i, j, k, iv, fy, occ, sv, ov, pv); });
+        for_face_column<1, COLUMN>(P, b - bu, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<1>(P, q, i, j, k, iv, fy, occ, sv, ov, pv); });
     } else {
-        for_face_column<2>(P, b - bu - bv, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<2>(P, q, i, j, k, iw, fz, occ, sw, ow, pw); });
+        for_face_column<2, COLUMN>(P, b - bu - bv, planes, [&](uint32_t q, int i, int j, int k) { face_force_one<2>(P, q, i, j, k, iw, fz, occ, sw, ow, pw); });
     }
 }
 
@@ -439,9 +439,10 @@ __global__ void __launch_bounds__(256) pad_ghost_kernel(const __grid_constant__ 
 
 // ------------------------------------------------------------------------------------------ pressure rhs
 // b = -(h^2/dt) div u* + sum of OUTFLOW face pressures; 0 at solid cells and at the anchor (:1304-1328).
+template <bool COLUMN>
 __global__ void __launch_bounds__(kThreads) rhs_kernel(const __grid_constant__ StepParams P, const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor, float* __restrict__ rhs, int planes) {
     pdl_begin();
-    for_column(P, planes, [&](uint32_t q, int x, int y, int z) {
+    for_column<COLUMN>(P, planes, [&](uint32_t q, int x, int y, int z) {
         // every load is issued before the anchor/solid test (the six faces of a cell always exist)
         const bool zero = static_cast<int32_t>(q) == __ldg(anchor) || occ[q] != 0;
         const float h = P.h;
@@ -513,16 +514,17 @@ __device__ __forceinline__ void project_one(const StepParams& P, uint32_t q, int
     }));
 }
 
+template <bool COLUMN>
 __global__ void __launch_bounds__(kThreads) project_kernel(const __grid_constant__ StepParams P, const float* __restrict__ iu, const float* __restrict__ iv, const float* __restrict__ iw, const float* __restrict__ p, const double* __restrict__ p64, const uint8_t* __restrict__ occ, const float* __restrict__ su, const float* __restrict__ sv, const float* __restrict__ sw, float* __restrict__ ou,
                                                             float* __restrict__ ov, float* __restrict__ ow, float* __restrict__ pu, float* __restrict__ pv, float* __restrict__ pw, unsigned bu, unsigned bv, int planes) {
     pdl_begin();
     const unsigned b = blockIdx.x;
     if (b < bu) {
-        for_face_column<0>(P, b, planes, [&](uint32_t q, int i, int j, int k) { project_one<0>(P, q, i, j, k, iu, p, p64, occ, su, ou, pu); });
+        for_face_column<0, COLUMN>(P, b, planes, [&](uint32_t q, int i, int j, int k) { project_one<0>(P, q, i, j, k, iu, p, p64, occ, su, ou, pu); });
     } else if (b < bu + bv) {
-        for_face_column<1>(P, b - bu, planes, [&](uint32_t q, int i, int j, int k) { project_one<1>(P, q, i, j, k, iv, p, p64, occ, sv, ov, pv); });
+        for_face_column<1, COLUMN>(P, b - bu, planes, [&](uint32_t q, int i, int j, int k) { project_one<1>(P, q, i, j, k, iv, p, p64, occ, sv, ov, pv); });
     } else {
-        for_face_column<2>(P, b - bu - bv, planes, [&](uint32_t q, int i, int j, int k) { project_one<2>(P, q, i, j, k, iw, p, p64, occ, sw, ow, pw); });
+        for_face_column<2, COLUMN>(P, b - bu - bv, planes, [&](uint32_t q, int i, int j, int k) { project_one<2>(P, q, i, j, k, iw, p, p64, occ, sw, ow, pw); });
     }
 }
 
@@ -833,9 +835,12 @@ bool set_advect_tile(StepParams& P, int code) {
 // Cells of a column per thread in the projection, face-force and right-hand-side kernels (for_column). They are bound
 // by instruction issue, a good part of it index arithmetic, which a column pays once: 256x384x256 face force 453 -> 333 us,
 // projection 365 -> 271, right-hand side 142 -> 119; 128^3 34 -> 30, 30 -> 25, 13 -> 10. Two cells
-// give half of that, 8 or 16 leave 97x141x83 too few threads (projection 20, 21, 26 and 41 us with 2, 4, 8 and 16). Below
-// kColumnCells (32^3 would keep 4 blocks busy) and on thin planes, which would fill their blocks badly, a thread takes one
-// cell. Vorticity and cell force got slower as columns (30 -> 40 and 22 -> 27 us at 97x141x83) and stay with one.
+// give half of that, 8 or 16 leave 97x141x83 too few threads (projection 20, 21, 26 and 41 us with 2, 4, 8 and 16).
+// Where the line lies: the three kernels together, with one cell against columns, take 34 and 46 us at 32^3, 25.6 and 28.1 at
+// 64^3, 29.9 and 28.6 at 72^3, 36.0 and 33.5 at 84^3, 38.1 and 34.5 at 88^3, 56 and 46 at 97x141x83. Columns win from about
+// 370 000 cells; the line at kColumnCells keeps to the sizes where they win by a tenth or more. Planes below kColumnSlab cells
+// would fill their blocks badly (16x16x2600 36.2 and 36.0). Vorticity and cell force got slower as
+// columns (30 -> 40 and 22 -> 27 us at 97x141x83) and stay with one.
 int column_planes(const StepParams& P) { return P.n >= kColumnCells && static_cast<uint32_t>(P.nx) * P.ny >= kColumnSlab ? std::max(kColumnPlanes, (P.nz + 65535) / 65535) : 0; }
 dim3 column_grid(const StepParams& P, int planes) { return planes > 0 ? dim3(blocks_for(static_cast<uint64_t>(P.nx) * P.ny), (P.nz + planes - 1) / planes) : dim3(blocks_for(P.n)); }
 
@@ -866,7 +871,7 @@ cudaError_t launch_cell_force(const StepParams& P, const float* wx, const float*
 cudaError_t launch_face_force(const StepParams& P, ConstFaces in, const float* fx, const float* fy, const float* fz, const uint8_t* occ, ConstFaces solid, Faces out, cudaStream_t s, Faces pad) {
     const int planes = column_planes(P);
     const FaceBlocks B = face_blocks(P, planes);
-    launch_pdl(face_force_kernel, B.grid, dim3(kThreads), 0, s, P, in.u, in.v, in.w, fx, fy, fz, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, B.u, B.v, planes);
+    launch_pdl(planes > 0 ? face_force_kernel<true> : face_force_kernel<false>, B.grid, dim3(kThreads), 0, s, P, in.u, in.v, in.w, fx, fy, fz, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, B.u, B.v, planes);
     return cudaGetLastError();
 }
 
@@ -936,14 +941,14 @@ cudaError_t launch_advect_velocity(const StepParams& P, ConstFaces in, ConstFace
 
 cudaError_t launch_rhs(const StepParams& P, ConstFaces vel, const uint8_t* occ, const int32_t* anchor, float* rhs, cudaStream_t s) {
     const int planes = column_planes(P);
-    launch_pdl(rhs_kernel, column_grid(P, planes), dim3(kThreads), 0, s, P, vel.u, vel.v, vel.w, occ, anchor, rhs, planes);
+    launch_pdl(planes > 0 ? rhs_kernel<true> : rhs_kernel<false>, column_grid(P, planes), dim3(kThreads), 0, s, P, vel.u, vel.v, vel.w, occ, anchor, rhs, planes);
     return cudaGetLastError();
 }
 
 cudaError_t launch_project(const StepParams& P, ConstFaces in, const float* pressure, const double* pressure64, const uint8_t* occ, ConstFaces solid, Faces out, cudaStream_t s, Faces pad) {
     const int planes = column_planes(P);
     const FaceBlocks B = face_blocks(P, planes);
-    launch_pdl(project_kernel, B.grid, dim3(kThreads), 0, s, P, in.u, in.v, in.w, pressure, pressure64, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, B.u, B.v, planes);
+    launch_pdl(planes > 0 ? project_kernel<true> : project_kernel<false>, B.grid, dim3(kThreads), 0, s, P, in.u, in.v, in.w, pressure, pressure64, occ, solid.u, solid.v, solid.w, out.u, out.v, out.w, pad.u, pad.v, pad.w, B.u, B.v, planes);
     return cudaGetLastError();
 }
 
