@@ -66,3 +66,46 @@ def test_solid_density_is_the_nearest_fluid_density(smoke_lib, cuda_stream, shap
     for z, y, x in zip(*np.nonzero(occ)):
         cell = nearest_fluid(occ, z, y, x, PERIODIC[boundary])
         assert density[z, y, x] == (0.0 if cell is None else density[cell]), (z, y, x, cell)
+
+
+# a cell by itself up to shell 1, a warp from shell 2 on: layers of one to six solid planes, half the cells at random
+@pytest.mark.parametrize("boundary", ["closed", "plume", "zout"])
+@pytest.mark.parametrize("kind", ["half", "layer1", "layer3", "layer4", "layer6"])
+def test_shallow_and_deep_solids(smoke_lib, cuda_stream, kind, boundary):
+    nz, ny, nx = 14, 9, 35
+    cfg = scenes.make_config(nx, ny, nz, boundary=boundary)
+    inp = scenes.random_inputs(cfg, seed=8, solids=False)
+    z = np.indices((nz, ny, nx))[0]
+    occ = np.random.default_rng(9).uniform(size=(nz, ny, nx)) < 0.5 if kind == "half" else (z >= 2) & (z < 2 + int(kind[5:]))
+    occ = inp["occupancy"] = occ.astype(np.uint8)
+    sim = smoke_b200.Simulation(smoke_lib, cfg, cuda_stream)
+    keep = scenes.load_gpu(sim, inp)
+    with torch.cuda.stream(cuda_stream):
+        sim.step()
+    density = sim.snapshot([abi.VIEW_DENSITY])["density"]
+    sim.close()
+    del keep
+    for c in zip(*np.nonzero(occ)):
+        assert density[c] == density[nearest_fluid(occ, *c, PERIODIC[boundary])], c
+
+
+def test_depth_beyond_a_32_bit_shell(smoke_lib, cuda_stream):
+    """Solids up to 13 750 cells deep in a line of cells: the whole shell of that radius has more than 2^32 cells, the part of it
+    inside the domain two. Ties go to the lower end (first in scan order)."""
+    n, low, high = 30000, 1000, 28501  # solid [low, high)
+    cfg = scenes.make_config(1, 1, n, boundary="closed")
+    inp = scenes.random_inputs(cfg, seed=10, solids=False)
+    occ = np.zeros((n, 1, 1), np.uint8)
+    occ[low:high] = 1
+    inp["occupancy"] = occ
+    sim = smoke_b200.Simulation(smoke_lib, cfg, cuda_stream)
+    keep = scenes.load_gpu(sim, inp)
+    with torch.cuda.stream(cuda_stream):
+        sim.step()
+    density = sim.snapshot([abi.VIEW_DENSITY])["density"].ravel()
+    sim.close()
+    del keep
+    z = np.arange(low, high)
+    source = np.where(z - (low - 1) <= high - z, low - 1, high)
+    assert density[low - 1] != density[high]
+    assert np.array_equal(density[z], density[source])

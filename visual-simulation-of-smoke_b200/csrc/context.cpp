@@ -157,7 +157,7 @@ struct SmokeSimulationContext_t {
         slots.push_back({reinterpret_cast<void**>(&codes), (n + 2) * sizeof(uint16_t)});
         slots.push_back({reinterpret_cast<void**>(&occupancy), n});
         slots.push_back({reinterpret_cast<void**>(&fill_list), n * sizeof(FillEntry)});
-        slots.push_back({reinterpret_cast<void**>(&fill_count), sizeof(uint32_t)});
+        slots.push_back({reinterpret_cast<void**>(&fill_count), kFillCounts * sizeof(uint32_t)});
         slots.push_back({reinterpret_cast<void**>(&anchor), sizeof(int32_t)});
         slots.push_back({reinterpret_cast<void**>(&control), sizeof(PcgControl)});
         if (const size_t words = pcg_exchange_bytes(pcg_shape.resident)) slots.push_back({reinterpret_cast<void**>(&pcg.exchange), words});

@@ -40,6 +40,7 @@ struct FillEntry {
     uint32_t cell;
     int32_t source;
 };
+constexpr uint32_t kFillCounts = 2;  // entries of the list; those of them with no fluid cell next to them
 
 StepParams make_params(const SmokeSimulationConfig& cfg);
 

@@ -666,8 +666,43 @@ __global__ void __launch_bounds__(kThreads) stencil_code_kernel(const __grid_con
     codes[q] = static_cast<uint16_t>(mask | (diag << 8) | kCodeActive);
 }
 
-// The solid cells, in no particular order, each without a source (a warp's cells take one slot range).
-__global__ void __launch_bounds__(kThreads) fill_list_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, FillEntry* __restrict__ list, uint32_t* __restrict__ count) {
+// Sources of FillEntry while the list is built: a cell whose 26 neighbours are all solid, and one without any fluid cell.
+constexpr int32_t kFillDeep = -2, kFillNone = -1;
+
+// v + d on a density axis of n cells, |d| < n, wrapped on a periodic one; false when there is no such cell.
+__device__ __forceinline__ bool fill_axis(int& v, int d, int n, int per) {
+    v += d;
+    if (v < 0) {
+        v += n;
+        return per != 0;
+    }
+    if (v >= n) {
+        v -= n;
+        return per != 0;
+    }
+    return true;
+}
+
+// Cells of the 3 x 3 x 3 neighbourhood (bit 9 (dz + 1) + 3 (dy + 1) + dx + 1) at squared distance d2.
+__host__ __device__ constexpr uint32_t fill_ring(int d2) {
+    uint32_t m = 0;
+    for (int i = 0; i < 27; ++i) {
+        const int dx = i % 3 - 1, dy = i / 3 % 3 - 1, dz = i / 9 - 1;
+        if (dx * dx + dy * dy + dz * dz == d2) m |= 1u << i;
+    }
+    return m;
+}
+
+// Nearest-fluid source of each solid cell (:1243-1290): first Chebyshev shell (radius 1, 2, ...) holding a fluid cell,
+// smallest squared distance in it, first in (dz, dy, dx) scan order on ties, density periodicity.
+// Three kernels split it by depth, because a warp per cell wastes lanes on a small shell and a thread per cell makes the deepest
+// cell a serial chain. Rebuilding everything that depends on the occupancy, with a thread per cell throughout, a warp per cell
+// throughout and split: a sphere of radius 12 in 96x128x96 564, 103 and 86 us; of radius 40 in 128^3 19.1, 8.1 and 3.6 ms; half
+// of 128^3 solid at random 228, 717 and 138 us; walls of 8 cells there 823, 2667 and 768 us, a floor of 32 68, 119 and 36 ms;
+// walls of one cell in 256^3 666, 986 and 398 us.
+// The first one lists the solid cells, in no particular order (a warp's cells take one slot range), with the sources that shell
+// 1 holds: thin walls and scattered solids end here, a thread per cell with its 26 loads in flight.
+__global__ void __launch_bounds__(kThreads) fill_list_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor_ptr, FillEntry* __restrict__ list, uint32_t* __restrict__ count) {
     pdl_begin();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
     const bool solid = q < P.n && occ[q] != 0;
@@ -676,97 +711,174 @@ __global__ void __launch_bounds__(kThreads) fill_list_kernel(const __grid_consta
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(count, static_cast<uint32_t>(__popc(solids)));
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (solid) list[base + __popc(solids & ((1u << lane) - 1u))] = FillEntry{q, -1};
-}
-
-// Cell i of the surface of the cube of radius r (24 r^2 + 2 of them): the two z faces, then the rings between them.
-__device__ __forceinline__ void shell_offset(uint32_t i, int r, int& dx, int& dy, int& dz) {
-    const uint32_t side = 2u * r + 1u, face = side * side;
-    if (i < 2u * face) {
-        const uint32_t k = i < face ? i : i - face, row = k / side;
-        dz = i < face ? -r : r;
-        dy = static_cast<int>(row) - r;
-        dx = static_cast<int>(k - row * side) - r;
-        return;
-    }
-    i -= 2u * face;
-    const uint32_t ring = 8u * r, layer = i / ring;
-    uint32_t k = i - layer * ring;
-    dz = static_cast<int>(layer) - r + 1;
-    if (k < 2u * side) {
-        dy = k < side ? -r : r;
-        dx = static_cast<int>(k < side ? k : k - side) - r;
-    } else {
-        k -= 2u * side;
-        dy = static_cast<int>(k >> 1) - r + 1;
-        dx = (k & 1u) ? r : -r;
-    }
-}
-
-constexpr int kFillBatch = 4;  // neighbours a lane looks at together
-
-// Nearest-fluid source of each solid cell (:1243-1290): first Chebyshev shell (radius 1, 2, ...) holding a fluid cell,
-// smallest squared distance in it, first in (dz, dy, dx) scan order on ties, density periodicity. A cell at depth r has
-// (2 r + 1)^3 neighbours to look at, one load latency after the other if a thread walks them, and the deepest cell decides
-// the time; so a warp takes a cell and its lanes share each shell. The scan order is part of the key that the lanes reduce.
-// A sphere of solid cells in 96 x 128 x 96: 452 us with a thread per cell, 42 with these two kernels.
-__global__ void __launch_bounds__(kThreads) fill_source_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, const int32_t* __restrict__ anchor_ptr, FillEntry* __restrict__ list, const uint32_t* __restrict__ count) {
-    pdl_begin();
-    if (*anchor_ptr >= static_cast<int32_t>(P.n)) return;  // no fluid cell exists
-    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kThreads / 32), entries = *count;
-    const int max_radius = imax(P.nx, imax(P.ny, P.nz));
-    for (uint32_t e = blockIdx.x * (kThreads / 32) + threadIdx.x / 32; e < entries; e += warps) {
+    int32_t source = kFillNone;
+    if (solid && *anchor_ptr < static_cast<int32_t>(P.n)) {  // at least one fluid cell exists
         int x, y, z;
-        cell_xyz(P, list[e].cell, x, y, z);
-        int32_t best = -1;
-        for (int r = 1; r <= max_radius && best < 0; ++r) {
-            const uint64_t cells = 24ull * r * r + 2ull;
-            int best_d2 = 0x7fffffff;
-            uint64_t best_order = ~0ull;
-            for (uint64_t i0 = lane; i0 < cells; i0 += 32u * kFillBatch) {
-                int d[kFillBatch][3];
-                int32_t cell[kFillBatch];  // -1: outside the domain or solid
+        cell_xyz(P, q, x, y, z);
+        int cx[3], cy[3], cz[3];
+        bool ox[3], oy[3], oz[3];
 #pragma unroll
-                for (int u = 0; u < kFillBatch; ++u) {
-                    const uint64_t i = i0 + 32u * u;
-                    shell_offset(static_cast<uint32_t>(i < cells ? i : 0u), r, d[u][0], d[u][1], d[u][2]);
-                    int c[3] = {x + d[u][0], y + d[u][1], z + d[u][2]};
-                    const int nn[3] = {P.nx, P.ny, P.nz};
-                    bool ok = i < cells;
+        for (int k = 0; k < 3; ++k) {
+            cx[k] = x;
+            cy[k] = y;
+            cz[k] = z;
+            ox[k] = fill_axis(cx[k], k - 1, P.nx, P.dper[0]);
+            oy[k] = fill_axis(cy[k], k - 1, P.ny, P.dper[1]);
+            oz[k] = fill_axis(cz[k], k - 1, P.nz, P.dper[2]);
+        }
+        uint32_t fluid = 0;
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        if (P.dper[a]) c[a] = wrapi(c[a], nn[a]);
-                        ok = ok && c[a] >= 0 && c[a] < nn[a];
-                    }
-                    cell[u] = ok ? static_cast<int32_t>(cidx(P, c[0], c[1], c[2])) : -1;
-                }
-                uint8_t solid[kFillBatch];
+        for (int i = 0; i < 27; ++i) {
+            if (i == 13) continue;
+            const int kx = i % 3, ky = i / 3 % 3, kz = i / 9;
+            if (ox[kx] && oy[ky] && oz[kz] && occ[cidx(P, cx[kx], cy[ky], cz[kz])] == 0) fluid |= 1u << i;
+        }
+        constexpr uint32_t kFaces = fill_ring(1), kEdges = fill_ring(2);
+        source = kFillDeep;
+        if (fluid != 0) {
+            const uint32_t nearest = (fluid & kFaces) ? fluid & kFaces : ((fluid & kEdges) ? fluid & kEdges : fluid);
+            const int i = __ffs(static_cast<int>(nearest)) - 1;
+            fill_axis(x, i % 3 - 1, P.nx, P.dper[0]);
+            fill_axis(y, i / 3 % 3 - 1, P.ny, P.dper[1]);
+            fill_axis(z, i / 9 - 1, P.nz, P.dper[2]);
+            source = static_cast<int32_t>(cidx(P, x, y, z));
+        }
+    }
+    if (solid) list[base + __popc(solids & ((1u << lane) - 1u))] = FillEntry{q, source};
+    const uint32_t deep = __ballot_sync(0xffffffffu, source == kFillDeep);
+    if (lane == 0 && deep != 0) atomicAdd(count + 1, static_cast<uint32_t>(__popc(deep)));
+}
+
+// The best cell of a shell so far: smallest squared distance, then first in scan order.
+struct FillBest {
+    long long d2;
+    int dz, dy, dx;
+    int32_t cell;
+    __device__ __forceinline__ void take(long long d, int z, int y, int x, int32_t c) {
+        const bool better = d != d2 ? d < d2 : (z != dz ? z < dz : (y != dy ? y < dy : x < dx));
+        if (!better) return;
+        d2 = d;
+        dz = z;
+        dy = y;
+        dx = x;
+        cell = c;
+    }
+};
+
+// A look at the two faces of the cube of radius r across axis A (0 x, 1 y, 2 z) around the cell at c, shared by W lanes: the z
+// faces whole, the y faces without their z edges, the x faces without any, so the three calls see each cell of the shell once.
+// Offsets that leave the domain are cut off beforehand, on a periodic axis at |d| < n: a longer one is a cell that a shorter one
+// has shown. A lane steps through rows and columns by W cells without a division.
+template <int A, int W>
+__device__ __forceinline__ void fill_faces(const StepParams& P, const uint8_t* __restrict__ occ, const int c[3], int r, uint32_t lane, FillBest& best) {
+    constexpr int R = A == 2 ? 1 : 2, C = A == 0 ? 1 : 0;  // axes of the rows and of the columns
+    const int n[3] = {P.nx, P.ny, P.nz};
+    const uint32_t stride[3] = {1u, static_cast<uint32_t>(P.nx), static_cast<uint32_t>(P.nx) * P.ny};
+    const int low[3] = {P.dper[0] ? 1 - P.nx : -c[0], P.dper[1] ? 1 - P.ny : -c[1], P.dper[2] ? 1 - P.nz : -c[2]};
+    const int high[3] = {P.dper[0] ? P.nx - 1 : P.nx - 1 - c[0], P.dper[1] ? P.ny - 1 : P.ny - 1 - c[1], P.dper[2] ? P.nz - 1 : P.nz - 1 - c[2]};
+    const bool minus = -r >= low[A], plus = r <= high[A];
+    if (!minus && !plus) return;
+    const int rr = A == 2 ? r : r - 1, rc = A == 0 ? r - 1 : r;
+    const int row0 = imax(-rr, low[R]), col0 = imax(-rc, low[C]);
+    const int rows = imin(rr, high[R]) - row0 + 1, cols = imin(rc, high[C]) - col0 + 1;
+    int at[2] = {c[A], c[A]};
+    fill_axis(at[0], minus ? -r : 0, n[A], P.dper[A]);
+    fill_axis(at[1], plus ? r : 0, n[A], P.dper[A]);
+    const uint32_t face[2] = {static_cast<uint32_t>(at[0]) * stride[A], static_cast<uint32_t>(at[1]) * stride[A]};
+    int row = W > 1 ? static_cast<int>(lane) / cols : 0, col = static_cast<int>(lane) - row * cols;
+    const int drow = W / cols, dcol = W - drow * cols;
+    constexpr int kBatch = 2;  // two cells of either face in flight
+    while (row < rows) {
+        uint32_t q[kBatch];
+        int d[kBatch][2];
+        uint8_t s[kBatch][2];
+        bool in[kBatch];
 #pragma unroll
-                for (int u = 0; u < kFillBatch; ++u) solid[u] = cell[u] >= 0 ? occ[cell[u]] : 1;
-#pragma unroll
-                for (int u = 0; u < kFillBatch; ++u) {
-                    if (solid[u]) continue;
-                    const int d2 = d[u][0] * d[u][0] + d[u][1] * d[u][1] + d[u][2] * d[u][2];
-                    const uint64_t order = (static_cast<uint64_t>(d[u][2] + r) << 42) | (static_cast<uint64_t>(d[u][1] + r) << 21) | static_cast<uint64_t>(d[u][0] + r);
-                    if (d2 < best_d2 || (d2 == best_d2 && order < best_order)) {
-                        best_d2 = d2;
-                        best_order = order;
-                        best = cell[u];
-                    }
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const int d2 = __shfl_xor_sync(0xffffffffu, best_d2, o);
-                const uint64_t order = __shfl_xor_sync(0xffffffffu, best_order, o);
-                const int32_t cell = __shfl_xor_sync(0xffffffffu, best, o);
-                if (d2 < best_d2 || (d2 == best_d2 && order < best_order)) {
-                    best_d2 = d2;
-                    best_order = order;
-                    best = cell;
-                }
+        for (int k = 0; k < kBatch; ++k) {
+            in[k] = row < rows;
+            d[k][0] = row0 + row;
+            d[k][1] = col0 + col;
+            int y = c[R], x = c[C];
+            fill_axis(y, d[k][0], n[R], P.dper[R]);
+            fill_axis(x, d[k][1], n[C], P.dper[C]);
+            q[k] = static_cast<uint32_t>(y) * stride[R] + static_cast<uint32_t>(x) * stride[C];
+            s[k][0] = in[k] && minus ? occ[face[0] + q[k]] : 1;
+            s[k][1] = in[k] && plus ? occ[face[1] + q[k]] : 1;
+            row += drow;
+            col += dcol;
+            if (col >= cols) {
+                col -= cols;
+                ++row;
             }
         }
-        if (lane == 0) list[e].source = best;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                if (s[k][side]) continue;
+                int o[3];
+                o[A] = side ? r : -r;
+                o[R] = d[k][0];
+                o[C] = d[k][1];
+                const long long d2 = static_cast<long long>(r) * r + static_cast<long long>(o[R]) * o[R] + static_cast<long long>(o[C]) * o[C];
+                best.take(d2, o[2], o[1], o[0], static_cast<int32_t>(face[side] + q[k]));
+            }
+    }
+}
+
+template <int W>
+__device__ __forceinline__ void fill_shell(const StepParams& P, const uint8_t* __restrict__ occ, const int c[3], int r, uint32_t lane, FillBest& best) {
+    fill_faces<2, W>(P, occ, c, r, lane, best);
+    fill_faces<1, W>(P, occ, c, r, lane, best);
+    fill_faces<0, W>(P, occ, c, r, lane, best);
+}
+__device__ __forceinline__ FillBest fill_nothing() { return FillBest{0x7fffffffffffffffll, 0, 0, 0, kFillNone}; }
+
+// From this many deep cells on, shells 2 to kFillNearRadius are searched by a thread per cell: all its lanes have work there,
+// a warp's do not (25, 15 and 9 cells a face in shell 2). With fewer, one thread's serial chain takes longer than the warps
+// do: the rebuild with threads and with warps there takes 90 and 77 us with 12 000 deep cells (a floor of 4 in 64^3), 106 and 112
+// with 28 000, 124 and 140 with 38 000, 190 and 260 with 77 000.
+constexpr uint32_t kFillMany = 32768;
+constexpr int kFillNearRadius = 4;
+__global__ void __launch_bounds__(kThreads) fill_near_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, FillEntry* __restrict__ list, const uint32_t* __restrict__ count) {
+    pdl_begin();
+    if (count[1] < kFillMany) return;
+    const uint32_t entries = count[0];
+    for (uint64_t e = blockIdx.x * kThreads + threadIdx.x; e < entries; e += static_cast<uint64_t>(gridDim.x) * kThreads) {
+        if (list[e].source != kFillDeep) continue;
+        int c[3];
+        cell_xyz(P, list[e].cell, c[0], c[1], c[2]);
+        FillBest best = fill_nothing();
+        for (int r = 2; r <= kFillNearRadius && best.cell < 0; ++r) fill_shell<1>(P, occ, c, r, 0u, best);
+        if (best.cell >= 0) list[e].source = best.cell;
+    }
+}
+
+// The deep cells that are left, a warp per cell, its lanes sharing each shell: a cell at depth r has
+// (2 r + 1)^3 neighbours to look at, one load latency after the other if a thread walks them, and the deepest cell decides the
+// time. A warp takes every warps-th entry, since deep cells lie together in the list.
+__global__ void __launch_bounds__(kThreads) fill_source_kernel(const __grid_constant__ StepParams P, const uint8_t* __restrict__ occ, FillEntry* __restrict__ list, const uint32_t* __restrict__ count) {
+    pdl_begin();
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kThreads / 32), entries = count[0];
+    const int max_radius = imax(P.nx, imax(P.ny, P.nz)), from = count[1] < kFillMany ? 2 : kFillNearRadius + 1;
+    if (count[1] == 0) return;
+    for (uint64_t first = blockIdx.x * (kThreads / 32) + threadIdx.x / 32; first < entries; first += 32ull * warps) {
+        const uint64_t e = first + static_cast<uint64_t>(lane) * warps;
+        FillEntry mine{0u, kFillNone};
+        if (e < entries) mine = list[e];
+        for (uint32_t deep = __ballot_sync(0xffffffffu, mine.source == kFillDeep); deep != 0; deep &= deep - 1u) {
+            const int owner = __ffs(static_cast<int>(deep)) - 1;
+            int c[3];
+            cell_xyz(P, __shfl_sync(0xffffffffu, mine.cell, owner), c[0], c[1], c[2]);
+            FillBest best = fill_nothing();
+            for (int r = from; r <= max_radius; ++r) {
+                fill_shell<32>(P, occ, c, r, lane, best);
+                if (__any_sync(0xffffffffu, best.cell >= 0)) break;
+            }
+            for (int o = 16; o > 0; o >>= 1)
+                best.take(__shfl_xor_sync(0xffffffffu, best.d2, o), __shfl_xor_sync(0xffffffffu, best.dz, o), __shfl_xor_sync(0xffffffffu, best.dy, o), __shfl_xor_sync(0xffffffffu, best.dx, o), __shfl_xor_sync(0xffffffffu, best.cell, o));
+            if (lane == static_cast<uint32_t>(owner)) list[e].source = best.cell;
+        }
     }
 }
 
@@ -988,12 +1100,14 @@ cudaError_t launch_stencil_codes(const StepParams& P, const uint8_t* occ, const 
 }
 
 cudaError_t launch_fill_build(const StepParams& P, const uint8_t* occ, const int32_t* anchor, FillEntry* list, uint32_t* count, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
+    cudaError_t e = cudaMemsetAsync(count, 0, kFillCounts * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    launch_pdl(fill_list_kernel, dim3(blocks_for(P.n)), dim3(kThreads), 0, s, P, occ, list, count);
+    launch_pdl(fill_list_kernel, dim3(blocks_for(P.n)), dim3(kThreads), 0, s, P, occ, anchor, list, count);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     constexpr unsigned kFillBlocks = 148 * 8;  // one resident wave; the entry count is on the device
-    launch_pdl(fill_source_kernel, dim3(std::min(kFillBlocks, blocks_for(P.n))), dim3(kThreads), 0, s, P, occ, anchor, list, static_cast<const uint32_t*>(count));
+    if (P.n > kFillMany) launch_pdl(fill_near_kernel, dim3(std::min(kFillBlocks, blocks_for(P.n))), dim3(kThreads), 0, s, P, occ, list, static_cast<const uint32_t*>(count));
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    launch_pdl(fill_source_kernel, dim3(std::min(kFillBlocks, blocks_for(P.n))), dim3(kThreads), 0, s, P, occ, list, static_cast<const uint32_t*>(count));
     return cudaGetLastError();
 }
 
