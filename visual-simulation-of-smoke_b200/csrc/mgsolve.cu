@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <set>
 #include <utility>
 
 #include "launch.h"
@@ -1617,10 +1618,24 @@ void launch_prolong(const MgHierarchy& H, int l, int depth, cudaStream_t s) {
     else launch_prolong_instance<false>(H, l, depth, s);
 }
 
+// Lets the block-level kernel take all of a block's shared memory, once per device: the limit belongs to the kernel, so a
+// context that set it to its own need would lower it under another thread's launch. (Where this fails, so does the launch.)
+void allow_block_bytes() {
+    static std::mutex lock;
+    static std::set<int> done;
+    int dev = 0, most = 0;
+    cudaFuncAttributes a{};
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> guard(lock);
+    if (!done.insert(dev).second) return;
+    if (cudaFuncGetAttributes(&a, mg_block_kernel) != cudaSuccess || cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return;
+    cudaFuncSetAttribute(mg_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - static_cast<int>(a.sharedSizeBytes));
+}
+
 // The block-level kernel, with its levels' cells in shared memory.
 void launch_block(const MgHierarchy& H, cudaStream_t s) {
     const uint32_t bytes = H.block_cells * kBlockCellBytes;
-    if (bytes > 48u * 1024u && cudaFuncSetAttribute(mg_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) != cudaSuccess) return;  // the caller reads the error
+    if (bytes > 48u * 1024u) allow_block_bytes();  // over 819 cells: nearly one-dimensional grids
     launch_pdl(mg_block_kernel, 1, kBlockLevelThreads, bytes, s, H);
 }
 
