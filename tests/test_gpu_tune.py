@@ -151,3 +151,15 @@ def test_autotune_restores_state_and_caches(smoke_lib):
     assert rep3["from_cache"] and rep3["chosen"] == rep["chosen"] and third.launch_tune() == rep["chosen"]
     for s in (sim, twin, third):
         s.close()
+
+
+@pytest.mark.parametrize("solver,grids", [((abi.SOLVER_FIXED_CG, abi.REDUCTION_FP32, 500, 1e-5, 0), 0), (JACOBI, (len(abi.PCG_GRID_NAMES) - 1) + (len(abi.PCG_REGS_NAMES) - 1))], ids=["on_chip", "streaming"])
+def test_autotune_times_only_shapes_that_the_solve_has(smoke_lib, solver, grids):
+    """A fixed-count solve that keeps its state on the chip ignores the streaming kernel's grid and register variant: timing them
+    would compare equal runs and could keep one by noise."""
+    sim, keep = make(smoke_lib, SHAPES[0], solver)
+    rep = sim.autotune(steps=1, force=True)
+    assert len(rep["records"]) == 1 + (len(abi.ADVECT_TILE_NAMES) - 1) + grids
+    if grids == 0:
+        assert all(r["pcg_grid"] == 0 and r["pcg_regs"] == 0 for r in rep["records"])
+    sim.close()

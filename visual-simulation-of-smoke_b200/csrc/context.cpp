@@ -979,7 +979,7 @@ SmokeSimulationResult smoke_b200_autotune_cuda(SmokeSimulationContext c, uint32_
                         t.mg_wave = v;
                         consider(t);
                     }
-            } else {
+            } else if (!pcg_runs_resident(c->pcg_settings(), c->pcg_shape, c->pcg)) {  // the resident kernel has no shapes to try
                 for (uint32_t v = 0; v < static_cast<uint32_t>(kPcgGridCount); ++v)
                     if (v != base_grid.pcg_grid) {
                         SmokeB200LaunchTune t = best.tune;
