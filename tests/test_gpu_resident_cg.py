@@ -49,6 +49,22 @@ def test_fixed_cg_in_one_cluster_matches_oracle(smoke_lib, cuda_stream, shape):
     check_against_oracle(smoke_lib, cuda_stream, shape, "plume", abi.REDUCTION_FP32)
 
 
+# 69, 70 (the most that a block holds) and 71 planes a block on 148 SMs; the last is the streaming kernel's
+@pytest.mark.parametrize("reduction", [abi.REDUCTION_FP32, abi.REDUCTION_FP64], ids=["fp32", "fp64"])
+@pytest.mark.parametrize("nz,on_chip", [(127, True), (128, True), (130, False)])
+def test_the_largest_grids_on_the_chip(smoke_lib, cuda_stream, nz, on_chip, reduction):
+    check_against_oracle(smoke_lib, cuda_stream, (128, 160, nz), "plume", reduction)
+    cfg = scenes.make_config(128, 160, nz, boundary="plume", pressure_iterations=10)
+    sim = smoke_b200.Simulation(smoke_lib, cfg, cuda_stream)
+    sim.set_solver(abi.SOLVER_FIXED_CG, reduction)
+    st = abi.SolverStatus()
+    # the hook takes the solves that run on the chip; a block that does not exist withholds nothing
+    rc = smoke_lib.lib.smoke_b200_test_exchange_timeout_cuda(sim.handle, 1 << 20, 1, 1000, C.byref(st))
+    sim.close()
+    assert (rc == abi.RESULT_OK) == on_chip
+    assert not on_chip or st.status == abi.SOLVE_ITERATION_CAP
+
+
 def check_against_oracle(smoke_lib, cuda_stream, shape, boundary, reduction):
     cfg = scenes.make_config(*shape, boundary=boundary, mode=abi.LINEAR, pressure_iterations=10)
     inp = scenes.random_inputs(cfg, seed=sum(shape), solids=shape[0] != 32)

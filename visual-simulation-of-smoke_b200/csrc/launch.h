@@ -152,7 +152,7 @@ struct PcgResidentPlan {
     uint32_t total;
     int blocks, planes;
 };
-constexpr int kPcgResidentPlanes = 70;  // 231,680 bytes of shared memory, and 140 registers for a thread's w and s
+constexpr int kPcgResidentPlanes = 70;  // 230,560 bytes of shared memory (272 more for the sums, of 232,448 that a block can have), and 140 registers for a thread's w and s
 PcgResidentPlan pcg_resident_plan(int nx, int ny, int nz, int sms);
 size_t pcg_exchange_bytes(const PcgResidentPlan& plan);
 

@@ -432,9 +432,8 @@ cudaError_t launch_variant(const StepParams& P, const PcgSettings& S, int g, con
     return S.fp64 ? launch_one<false, double, MINB>(P, S, g, codes, b, x, work, ctl, s) : launch_one<false, float, MINB>(P, S, g, codes, b, x, work, ctl, s);
 }
 
-// Fixed-count solves of grids that fit on the chip run there (FP64 sums take 2 KB of shared memory, the space of the last
-// plane).
-bool pcg_runs_resident(const PcgSettings& S, const PcgLaunchShape& shape, const PcgWork& work) { return S.fixed && !S.jacobi && shape.resident.blocks > 0 && work.exchange != nullptr && (!S.fp64 || shape.resident.planes < kPcgResidentPlanes); }
+// Fixed-count solves of grids that fit on the chip run there.
+bool pcg_runs_resident(const PcgSettings& S, const PcgLaunchShape& shape, const PcgWork& work) { return S.fixed && !S.jacobi && shape.resident.blocks > 0 && work.exchange != nullptr; }
 
 cudaError_t launch_pcg(const StepParams& P, const PcgSettings& S, const PcgLaunchShape& shape, const uint16_t* codes, const float* b, float* x, PcgWork work, PcgControl* ctl, cudaStream_t s) {
     // the launch shape's knobs are this file's kernel's

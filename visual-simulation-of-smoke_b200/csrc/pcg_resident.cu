@@ -99,7 +99,9 @@ struct ResidentArgs {
 };
 
 // Shared memory of a block of `planes` planes in up to two column segments: r with its halo, p, the side halo's s, codes.
-inline uint32_t resident_smem(int planes) { return static_cast<uint32_t>(4 * (kSlab * (planes + 4) + (kThreads + kSideWords) * planes) + 2 * kThreads * planes); }
+constexpr uint32_t resident_smem(int planes) { return static_cast<uint32_t>(4 * (kSlab * (planes + 4) + (kThreads + kSideWords) * planes) + 2 * kThreads * planes); }
+
+static_assert(resident_smem(kPcgResidentPlanes) + 272u <= 227u * 1024u, "the largest block and its sums (FP64) fit");
 
 // A halo cell's s and r, formed from the w its owner published, must be the owner's bit for bit, so every rounding of the
 // recurrences is spelled out. (With the products left to the compiler's contraction the copies drifted apart by an ulp an
