@@ -66,3 +66,37 @@ def test_batch_rejects_duplicates_and_empty(smoke_lib, cuda_stream):
     assert smoke_lib.lib.smoke_b200_batch_create_cuda(twice, 0, None, C.byref(out)) == abi.RESULT_BACKEND_FAILURE
     assert smoke_lib.lib.smoke_b200_batch_destroy_cuda(None) == abi.RESULT_OK
     sim.close()
+
+
+# 60, 148 and 148 blocks of the on-chip fixed-count solve, each a cooperative launch whose blocks wait for one another
+LARGE = [dict(shape=(64, 48, 40), boundary="plume", mode=abi.LINEAR, seed=8), dict(shape=(72, 72, 72), boundary="closed", mode=abi.LINEAR, seed=9), dict(shape=(96, 96, 96), boundary="zout", mode=abi.LINEAR, seed=10)]
+FIXED = (abi.SOLVER_FIXED_CG, abi.REDUCTION_FP32, 500, 1e-5, 0)
+
+
+@pytest.mark.parametrize("form", ["batch", "streams"])
+def test_cooperative_solves_side_by_side(smoke_lib, form):
+    """In one batch graph, or on streams of their own, solves that need most of the chip each end as they do alone."""
+    alone = [make(smoke_lib, torch.cuda.Stream(), m, FIXED) for m in LARGE]
+    beside = [make(smoke_lib, torch.cuda.Stream(), m, FIXED) for m in LARGE]
+    steps = 4
+    for sim, _ in alone:
+        for _ in range(steps):
+            sim.step()
+        sim.stream.synchronize()
+    if form == "batch":
+        with smoke_b200.Batch([s for s, _ in beside]) as batch:
+            for _ in range(steps):
+                batch.step()
+            torch.cuda.synchronize()
+    else:
+        for _ in range(steps):
+            for sim, _ in beside:
+                sim.step()
+        torch.cuda.synchronize()
+    for (a, _), (b, _) in zip(alone, beside):
+        assert a.solver_status().status == b.solver_status().status == abi.SOLVE_ITERATION_CAP
+        ra, rb = a.snapshot(KINDS), b.snapshot(KINDS)
+        for key in ra:
+            assert scenes.rel_err(rb[key], ra[key]) < TOL, key
+    for s, _ in alone + beside:
+        s.close()

@@ -119,3 +119,31 @@ def test_halo_wait_that_runs_out_aborts_the_solve(smoke_lib, cuda_stream, shape,
     assert hook(sim.handle, block, 1, 100, C.byref(st)) == abi.RESULT_BACKEND_FAILURE  # no exchange of faces there
     sim.close()
     del keep
+
+
+@pytest.mark.parametrize("shape,boundary", [((8, 8, 8), "closed"), ((32, 8, 40), "plume"), ((40, 24, 9), "zout"), ((33, 41, 37), "closed"), ((64, 64, 64), "plume")])
+@pytest.mark.parametrize("reduction", [abi.REDUCTION_FP32, abi.REDUCTION_FP64], ids=["fp32", "fp64"])
+def test_the_two_kernels_agree_after_64_iterations(smoke_lib, cuda_stream, shape, boundary, reduction):
+    """The allocation-free solve runs the streaming kernel on the same system. The kernels' totals differ by the order in which up
+    to 148 FP64 partials are added (2^-53 each), which changes alpha or beta, rounded to FP32, only where the total lies that
+    close to a rounding boundary. Were one to flip in every one of 64 iterations (2^-24 of a step), with the growth by a factor
+    of ten allowed above, that would be 64 * 6e-8 * 10 < 1e-4 of the largest pressure."""
+    cfg = scenes.make_config(*shape, boundary=boundary, mode=abi.LINEAR, pressure_iterations=64)
+    inp = scenes.random_inputs(cfg, seed=sum(shape), solids=False)
+    sim = smoke_b200.Simulation(smoke_lib, cfg, cuda_stream)
+    keep = scenes.load_gpu(sim, inp)
+    sim.set_solver(abi.SOLVER_FIXED_CG, reduction)
+    with torch.cuda.stream(cuda_stream):
+        sim.step_stages(abi.STAGE_PRESSURE)
+        rhs = sim.view(abi.VIEW_FLOW_PRESSURE_RHS).clone()
+    p = sim.snapshot([abi.VIEW_FLOW_PRESSURE])["pressure"]
+    sim.close()
+    del keep
+    solve = smoke_lib.lib.smoke_b200_solve_pressure_noalloc_cuda
+    solve.argtypes = [C.POINTER(abi.Config), C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(abi.SolverDesc), C.c_void_p, C.POINTER(abi.SolverStatus)]
+    solve.restype = C.c_int
+    out, st, desc = torch.empty_like(rhs), abi.SolverStatus(), abi.SolverDesc(abi.SOLVER_FIXED_CG, reduction, 500, 1e-5, 0, 0)
+    torch.cuda.synchronize()
+    rc = solve(C.byref(cfg), None, C.c_void_p(rhs.data_ptr()), C.c_void_p(out.data_ptr()), C.byref(desc), C.c_void_p(cuda_stream.cuda_stream), C.byref(st))
+    assert rc == abi.RESULT_OK and st.iterations == 64
+    assert scenes.rel_err(p, out.cpu().numpy()) < 1e-4
