@@ -252,8 +252,8 @@ SMOKE_SIMULATION_API SmokeSimulationResult smoke_b200_solve_pressure_eager_cuda(
 SMOKE_SIMULATION_API SmokeSimulationResult smoke_b200_test_barrier_timeout_cuda(SmokeSimulationContext context, uint32_t block, uint32_t timeout_ms, SmokeB200SolverStatus* out_status);
 
 /* The same for a solve that keeps its state on the chip (FIXED_CG on grids that fit there; other solves are refused): block
- * `block` runs, but its neighbours never get its faces of exchange `exchange` (1: the start's; iteration i reads those of
- * exchange i, so pressure_iterations is the last that anything waits for). Their halo waits run out and the solve aborts with
+ * `block` runs, but never gets its neighbours' faces of exchange `exchange` (1: the start's; iteration i reads those of
+ * exchange i, so pressure_iterations is the last that anything waits for). Its halo waits run out and the solve aborts with
  * SMOKE_B200_SOLVE_BARRIER_TIMEOUT. A block or an exchange that does not exist withholds nothing. */
 SMOKE_SIMULATION_API SmokeSimulationResult smoke_b200_test_exchange_timeout_cuda(SmokeSimulationContext context, uint32_t block, uint32_t exchange, uint32_t timeout_ms, SmokeB200SolverStatus* out_status);
 

@@ -91,7 +91,7 @@ def check_against_oracle(smoke_lib, cuda_stream, shape, boundary, reduction):
 @pytest.mark.parametrize("exchange", [1, 5, 10])
 @pytest.mark.parametrize("shape,block", [((32, 8, 40), 2), ((48, 40, 32), 1), ((96, 96, 96), 70)], ids=["cluster", "grid", "planes24"])
 def test_halo_wait_that_runs_out_aborts_the_solve(smoke_lib, cuda_stream, shape, block, exchange):
-    """A block whose neighbours never get its faces of one exchange: their bounded waits run out, every block leaves, the
+    """A block that never gets its neighbours' faces of one exchange: its bounded waits run out, every block leaves, the
     status says so, and the next solve on the context gives the bits of the one before."""
     cfg = scenes.make_config(*shape, boundary="plume", mode=abi.LINEAR, pressure_iterations=10)
     inp = scenes.random_inputs(cfg, seed=sum(shape), solids=False)

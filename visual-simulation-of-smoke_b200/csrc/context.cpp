@@ -499,7 +499,7 @@ cudaError_t copy_or_zero(float* dst, const float* src, size_t count, cudaStream_
     return cudaMemcpyAsync(dst, src, count * sizeof(float), cudaMemcpyDeviceToDevice, s);
 }
 
-// The context's persistent solve with a block withheld (exchange > 0: only its faces of that exchange), and its status.
+// The context's persistent solve with a block withheld (exchange > 0: only the faces of that exchange, from it), and its status.
 SmokeSimulationResult solve_withheld(SmokeSimulationContext_t& c, uint32_t block, uint32_t exchange, uint32_t timeout_ms, SmokeB200SolverStatus* out) {
     PcgSettings S = c.pcg_settings();
     S.withhold_block = static_cast<int32_t>(block) + 1;

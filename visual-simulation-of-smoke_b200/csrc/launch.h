@@ -105,7 +105,7 @@ struct PcgSettings {
     int32_t warm_start;      // start from x instead of 0
     int32_t withhold_block;  // test only: > 0 makes block withhold_block - 1 leave before its first grid barrier
     uint32_t barrier_timeout_ms;  // bound of every grid-barrier wait (0: the default, 2000 ms)
-    int32_t withhold_exchange;  // test only, resident kernel: > 0 lets that block run and withhold its faces of this exchange
+    int32_t withhold_exchange;  // test only, resident kernel: > 0 lets that block run, but not see the faces of this exchange
 };
 
 struct PcgStatusDevice {

@@ -152,8 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     __shared__ double all[kPcgSumCopies][kSums];
     __shared__ int flag[2];  // a halo wait, a sum wait of this block gave up
     // test hook: this block never publishes, so the others' bounded waits run out and abort the solve
-    const bool withheld = A.withhold_block > 0 && static_cast<int>(blockIdx.x) == A.withhold_block - 1;
-    if (withheld && A.withhold_exchange == 0) return;
+    if (A.withhold_block > 0 && static_cast<int>(blockIdx.x) == A.withhold_block - 1 && A.withhold_exchange == 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;  // a warp is a row of the column
     const uint32_t G = gridDim.x, total = A.plan.total;
     const uint32_t ua = static_cast<uint32_t>((static_cast<uint64_t>(blockIdx.x) * total) / G);
@@ -303,6 +302,8 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
             // the halo's w were published before the sums that set alpha and beta: the z faces' and the first group of the side
             // faces' are in flight while the own cells advance
             unsigned long long zv[2][2], v[kItems];
+            // test hook: in one iteration (from 1) one block waits for faces with a tag that none carries
+            const uint32_t tag = A.withhold_exchange == it + 1 && static_cast<int>(blockIdx.x) == A.withhold_block - 1 ? phase ^ 0x80000000u : phase;
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                     const int zs = halo_slot(k, top);
                     if (zs < 0) continue;
                     if (M > 9) zv[k][top] = get_word(z_words(zs));
-                    if (tag_of(zv[k][top]) != phase) zv[k][top] = poll(z_words(zs), phase, halo_wait);
+                    if (tag_of(zv[k][top]) != tag) zv[k][top] = poll(z_words(zs), tag, halo_wait);
                     advance(__uint_as_float(static_cast<uint32_t>(zv[k][top])), fa, fb, sz[k][top], rs[z_plane(k, top) * kSlab + slot]);
                 }
             for (int j0 = j1; j0 < 3 * m; j0 += kItems * kWarps) {
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                     int word, rslot, hslot;
                     const int col = side_item(j, word, rslot, hslot);
                     if (col < 0) continue;
-                    if (tag_of(v[n]) != phase) v[n] = poll(side_words(col, plane_z(j / 3)) + word, phase, halo_wait);
+                    if (tag_of(v[n]) != tag) v[n] = poll(side_words(col, plane_z(j / 3)) + word, tag, halo_wait);
                     advance(__uint_as_float(static_cast<uint32_t>(v[n])), fa, fb, hs[hslot], rs[rslot]);
                 }
             }
@@ -368,8 +369,6 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
         // w = A r of the own cells, the faces' w published under a new tag; this thread's (r, r) and (w, r) in plane order
         T loc[kSums] = {0, 0};
         ++phase;
-        // test hook: the faces of one exchange (1: the start's) carry a tag that no reader waits for
-        const uint32_t face_tag = withheld && A.withhold_exchange == (first ? 1 : it + 2) ? phase - 1u : phase;
         {
             unsigned long long* const out = side_words(col0, za);  // units are consecutive: plane i's words 80 i further
             const float* r = ra;
@@ -392,8 +391,8 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                     w[i] = v;
                     loc[0] += static_cast<T>(r0) * static_cast<T>(r0);
                     loc[1] += static_cast<T>(v) * static_cast<T>(r0);
-                    if (yw >= 0) put_word(out + i * kSideWords + yw, __float_as_uint(v), face_tag);
-                    if (xw >= 0) put_word(out + i * kSideWords + xw, __float_as_uint(v), face_tag);
+                    if (yw >= 0) put_word(out + i * kSideWords + yw, __float_as_uint(v), phase);
+                    if (xw >= 0) put_word(out + i * kSideWords + xw, __float_as_uint(v), phase);
                 }
                 rm1 = r0;
                 r0 = r1;
@@ -407,15 +406,15 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
             for (int k = 0; k < 2; ++k) {
                 if (!owns(k)) continue;
                 const int lo = k == 0 ? 0 : m0, hi = k == 0 ? m0 - 1 : m - 1;
-                if (lo == 0 && za > 0) put_word(z_words(2 * blockIdx.x), value(lo), face_tag);
-                if (hi == m - 1 && plane_z(hi) < A.nz - 1) put_word(z_words(2 * blockIdx.x + 1), value(hi), face_tag);
-                if (A.per[2] && plane_z(lo) == 0) put_word(z_words(col_slot(col0 + k, 0)), value(lo), face_tag);
-                if (A.per[2] && plane_z(hi) == A.nz - 1) put_word(z_words(col_slot(col0 + k, 1)), value(hi), face_tag);
+                if (lo == 0 && za > 0) put_word(z_words(2 * blockIdx.x), value(lo), phase);
+                if (hi == m - 1 && plane_z(hi) < A.nz - 1) put_word(z_words(2 * blockIdx.x + 1), value(hi), phase);
+                if (A.per[2] && plane_z(lo) == 0) put_word(z_words(col_slot(col0 + k, 0)), value(lo), phase);
+                if (A.per[2] && plane_z(hi) == A.nz - 1) put_word(z_words(col_slot(col0 + k, 1)), value(hi), phase);
                 if (!thin) continue;
                 const Column& c = k == 0 ? c0 : c1;
                 for (int i = lo; i <= hi; ++i) {
-                    if (c.ey == 1 && c.north >= 0) put_word(out + i * kSideWords + CX + lane, value(i), face_tag);
-                    if (c.ex == 1 && c.east >= 0) put_word(out + i * kSideWords + 2 * CX + CY + warp, value(i), face_tag);
+                    if (c.ey == 1 && c.north >= 0) put_word(out + i * kSideWords + CX + lane, value(i), phase);
+                    if (c.ex == 1 && c.east >= 0) put_word(out + i * kSideWords + 2 * CX + CY + warp, value(i), phase);
                 }
             }
         }
