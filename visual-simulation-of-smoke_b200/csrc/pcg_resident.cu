@@ -59,8 +59,8 @@ __device__ __forceinline__ void get_words(const unsigned long long* p, unsigned 
 __device__ __forceinline__ uint32_t tag_of(unsigned long long v) { return static_cast<uint32_t>(v >> 32); }
 
 // A wait's bound, and where giving up is recorded: the grid's abort word and the block's flag for waits of this kind. Halo
-// waits and sum waits have a flag each: it is read behind the barrier that ends the waits, and another barrier comes before the
-// next waits that may set it, so every warp of the block reads the same value.
+// waits and sum waits have a flag each, read behind a barrier after those waits and before a barrier that comes before the next
+// ones of the kind, so every warp of the block reads the same value.
 struct Wait {
     PcgControl* ctl;
     int* flag;
@@ -367,12 +367,6 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
                 }
             }
             __syncthreads();
-            // r's halo is incomplete: leave without publishing, so that no block gets sums formed from it, in the last iteration
-            // either, after which nothing but those sums is waited for
-            if (*static_cast<volatile int*>(&flag[0]) != 0) {
-                status = SMOKE_B200_SOLVE_BARRIER_TIMEOUT;
-                break;
-            }
         }
         // w = A r of the own cells, the faces' w published under a new tag; this thread's (r, r) and (w, r) in plane order
         T loc[kSums] = {0, 0};
@@ -433,6 +427,9 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
             if (lane == 0) red[k][warp] = v;
         }
         __syncthreads();
+        // a block whose halo is incomplete publishes no sums: no other block takes any that were formed from it, in the last
+        // iteration either, after which nothing but those sums is waited for
+        const bool halo_failed = *static_cast<volatile int*>(&flag[0]) != 0;
         if (warp == 0) {
             // 8 lanes per sum add the warps' partials; lanes 0 and 1 of them write the two halves
             static_assert(kWarps == 8 && kSums == 2, "8 lanes per sum");
@@ -441,7 +438,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
             const double mine = static_cast<double>(t);
-            if (lane < 16 && part < 2) put_word(sum_words(blockIdx.x) + 2 * k + part, part ? __double2hiint(mine) : __double2loint(mine), phase);
+            if (lane < 16 && part < 2 && !halo_failed) put_word(sum_words(blockIdx.x) + 2 * k + part, part ? __double2hiint(mine) : __double2loint(mine), phase);
         }
         if (!first) {
             // while the other blocks' words travel: x += alpha p
@@ -500,7 +497,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
         for (int c = 0; c < kPcgSumCopies; ++c)
 #pragma unroll
             for (int k = 0; k < kSums; ++k) sums[k] += static_cast<T>(all[c][k]);
-        if (*static_cast<volatile int*>(&flag[1]) != 0) {
+        if (halo_failed || *static_cast<volatile int*>(&flag[1]) != 0) {
             status = SMOKE_B200_SOLVE_BARRIER_TIMEOUT;
             break;
         }
