@@ -22,6 +22,12 @@ namespace {
 constexpr int kThreads = 256;
 
 inline unsigned blocks_for(uint64_t count, int threads = kThreads) { return static_cast<unsigned>((count + threads - 1) / threads); }
+// SMs of the current device (1 where it cannot be read: the launch then reports why).
+inline unsigned sm_count() {
+    int dev = 0, sms = 1;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1u;
+    return static_cast<unsigned>(sms);
+}
 
 // The step's elementwise kernels call f(q, x, y, z), q linear, for one cell per thread, kThreads consecutive ones per block, or
 // (COLUMN) for `planes` cells of a column (x, y): block blockIdx.x takes kThreads consecutive cells of a plane, blockIdx.y a run
@@ -609,10 +615,9 @@ __global__ void set_int_kernel(int32_t* p, int32_t v) {
     *p = v;
 }
 
-// anchor = smallest fluid cell index (:1292-1302); warp minimum first, one atomic per warp.
-// The first fluid cell into *anchor (set to n before). Warps take runs of 32 cells in ascending order and stop at the first
-// one with a fluid cell or past an anchor already found, so a grid of one block per SM reads little more than the cells up to
-// it (one atomic for each of the grid's warps took 25 us at 96x128x96, now 2.4).
+// anchor = smallest fluid cell index (:1292-1302), into *anchor (set to n before). Warps take runs of 32 cells in ascending
+// order and stop at the first one with a fluid cell or past an anchor already found, so a grid of one block per SM reads little
+// more than the cells up to it (one atomic for each of the grid's warps took 25 us at 96x128x96, now 2.4).
 __global__ void __launch_bounds__(kThreads) anchor_kernel(uint32_t n, const uint8_t* __restrict__ occ, int32_t* anchor) {
     pdl_begin();
     const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kThreads / 32);
@@ -1090,7 +1095,7 @@ cudaError_t launch_occupancy_float(const StepParams& P, const uint8_t* occ, floa
 
 cudaError_t launch_anchor(const StepParams& P, const uint8_t* occ, int32_t* anchor, cudaStream_t s) {
     launch_pdl(set_int_kernel, dim3(1), dim3(1), 0, s, anchor, static_cast<int32_t>(P.n));
-    launch_pdl(anchor_kernel, dim3(std::min(148u, blocks_for(P.n))), dim3(kThreads), 0, s, P.n, occ, anchor);
+    launch_pdl(anchor_kernel, dim3(std::min(sm_count(), blocks_for(P.n))), dim3(kThreads), 0, s, P.n, occ, anchor);
     return cudaGetLastError();
 }
 
@@ -1104,10 +1109,10 @@ cudaError_t launch_fill_build(const StepParams& P, const uint8_t* occ, const int
     if (e != cudaSuccess) return e;
     launch_pdl(fill_list_kernel, dim3(blocks_for(P.n)), dim3(kThreads), 0, s, P, occ, anchor, list, count);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    constexpr unsigned kFillBlocks = 148 * 8;  // one resident wave; the entry count is on the device
-    if (P.n > kFillMany) launch_pdl(fill_near_kernel, dim3(std::min(kFillBlocks, blocks_for(P.n))), dim3(kThreads), 0, s, P, occ, list, static_cast<const uint32_t*>(count));
+    const dim3 wave(std::min(sm_count() * 8u, blocks_for(P.n)));  // 8 blocks an SM; the entry count is on the device
+    if (P.n > kFillMany) launch_pdl(fill_near_kernel, wave, dim3(kThreads), 0, s, P, occ, list, static_cast<const uint32_t*>(count));
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    launch_pdl(fill_source_kernel, dim3(std::min(kFillBlocks, blocks_for(P.n))), dim3(kThreads), 0, s, P, occ, list, static_cast<const uint32_t*>(count));
+    launch_pdl(fill_source_kernel, wave, dim3(kThreads), 0, s, P, occ, list, static_cast<const uint32_t*>(count));
     return cudaGetLastError();
 }
 
