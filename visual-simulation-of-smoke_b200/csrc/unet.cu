@@ -629,7 +629,6 @@ __global__ void __launch_bounds__(kEpiThreads) wgrad_kernel(const __grid_constan
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
     pdl_trigger();  // after the allocation: a later kernel's block must not take the tensor memory that one of ours still asks for
-    pdl_wait();  // the set-up above overlaps the previous kernel's tail
     constexpr uint32_t idesc = tc::idesc_bf16_f32(128, GN, true, true);
     const uint32_t a_base = tc::smem_addr(As), b_base = tc::smem_addr(Bs);
     const uint32_t chunks = (a.n + kWgradCells - 1) / kWgradCells;
