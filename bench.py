@@ -275,8 +275,8 @@ MG_BYTES_PER_CELL_ITERATION = 85.0
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum over every kernel) of one multigrid FCG solve from zero
 # on the 128^3 plume after the spin-up, 12 iterations, 1 pass: the kernels of the graph launched one by one
 # (bench.py --profile solve, ncu --cache-control none so that L2 carries over between kernels as in the graph);
-# 63.8 MB read + 447.9 MB written, per grid size. Scaled by iterations when a solve takes another count.
-MG_SOLVE_DRAM_BYTES = {128: (511.7e6, 12)}
+# 73.7 MB read + 436.6 MB written, per grid size. Scaled by iterations when a solve takes another count.
+MG_SOLVE_DRAM_BYTES = {128: (510.3e6, 12)}
 
 
 def solver_kernel_roofline(sim, n_cells, peak_gbs, peak_kind, repeats=5, bytes_per_iteration=JACOBI_BYTES_PER_CELL_ITERATION, kernel="pcg_kernel", traffic_table=None):
